@@ -10,11 +10,11 @@
 // whose sizes are read on the device, with no host synchronisation inside a
 // render call.
 //
-// Path state is indexed by a stable path id (pid = s * npix + pixel) and the
-// queues hold path ids, so a path keeps its RNG stream and its radiance
-// accumulator wherever it is queued. Each path accumulates its own radiance;
-// the resolve adds paths to their pixel in sample order, so the image does not
-// depend on queue order, wave size, or what else is rendered alongside.
+// A path has a stable id (pid = s * npix + pixel) that fixes its RNG stream and
+// its radiance accumulator wherever it is queued; its ray and throughput move
+// with its queue entry. Each path accumulates its own radiance; the resolve
+// adds paths to their pixel in sample order, so the image does not depend on
+// queue order, wave size, or what else is rendered alongside.
 #include <algorithm>
 #include <cstddef>
 #include <cstring>
@@ -28,7 +28,14 @@ namespace {
 
 using namespace sh;
 
-constexpr uint32_t kFlagSpecular = 1u;
+constexpr uint64_t kSampleStride = 0x9E3779B97F4A7C15ull;  // between the RNG seeds of a pixel's samples
+constexpr uint32_t kSpecularBit = 0x80000000u;  // of thr.w
+constexpr float kCameraTmin = 0.0f, kCameraTmax = 1e34f;
+constexpr float kScatterTmin = 1e-4f, kScatterTmax = 1e38f;
+constexpr float kShadowTmin = 0.0f, kShadowTmax = 0.9999f;
+// Draws of a path's RNG: 2 for the camera jitter, then per bounce 1 for roulette
+// (from bounce 1 on) and 8 for shading.
+inline uint32_t draws_before(int b) { return b == 0 ? 2u : 9u * (uint32_t)b + 1u; }
 constexpr int kShadeThreads = 256;
 constexpr int kShadowBase = kMaxDepth + 1;  // shadow queue counters start here
 constexpr int kErrWord = 2 * kMaxDepth + 4;
@@ -296,7 +303,7 @@ __global__ void __launch_bounds__(kShadeThreads) k_camera(Paths ps) {
         const uint32_t pixel = local % J.npix;
         const uint32_t s = J.sample_base + local / J.npix;
         const uint64_t inc = pcg_inc(pixel);
-        uint64_t st = pcg_seed(J.seed + (uint64_t)s * 0x9E3779B97F4A7C15ull, inc);
+        uint64_t st = pcg_seed(J.seed + (uint64_t)s * kSampleStride, inc);
         const float j0 = pcg_float(st, inc), j1 = pcg_float(st, inc);
         const DevCamera& c = J.sc.cam;
         const float rx = (float)(pixel % c.width) + j0;
@@ -306,36 +313,45 @@ __global__ void __launch_bounds__(kShadeThreads) k_camera(Paths ps) {
         const V3 d = normalize(v3(c.m[0] * dc.x + c.m[1] * dc.y + c.m[2] * dc.z,
                                   c.m[4] * dc.x + c.m[5] * dc.y + c.m[6] * dc.z,
                                   c.m[8] * dc.x + c.m[9] * dc.y + c.m[10] * dc.z));
-        ps.ray[2ull * pid] = make_float4(c.m[3], c.m[7], c.m[11], d.x);
-        ps.ray[2ull * pid + 1] = make_float4(d.y, d.z, 0.0f, 1e34f);
-        ps.thr[pid] = make_float4(1.0f, 1.0f, 1.0f, 0.0f);
-        ps.acc[pid] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        ps.flags[pid] = 0;
-        ps.job[pid] = j;
-        ps.rng[pid] = st;
-        ps.qa[pid] = pid;
+        ps.ray[0][2ull * pid] = make_float4(c.m[3], c.m[7], c.m[11], d.x);
+        ps.ray[0][2ull * pid + 1] = make_float4(d.y, d.z, __uint_as_float(pid), __uint_as_float(j));
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) ps.cnt[0] = h.total_paths;
 }
 
 // ---- traversal over queues ----------------------------------------------------------
+// The BVH of a job's rays: nodes, triangles and root (the 8-wide root is node 0
+// of a scene with triangles, known without reading the BVH's header).
+template <int LAYOUT>
+__device__ __forceinline__ uint32_t job_bvh(const JobDev* jobs, uint32_t j, const void*& nd, const Tri*& tr) {
+    const SceneDev& sc = jobs[j].sc;
+    nd = sc.nodes;
+    tr = sc.tris;
+    if (LAYOUT == kLayoutBvh8Q8) return sc.num_tris ? 0u : kNoNode;
+    return sc.meta->root;
+}
+
+template <int LAYOUT>
 struct QueueSrc {
-    const uint32_t* __restrict__ q;
-    const Paths* ps;
-    uint64_t n;
-    __device__ __forceinline__ uint32_t load(uint64_t i, float4& r0, float4& r1, const void*& nd, const Tri*& tr) const {
-        const uint32_t pid = q[i];
-        r0 = ps->ray[2ull * pid];
-        r1 = ps->ray[2ull * pid + 1];
-        const SceneDev& sc = ps->jobs[ps->job[pid]].sc;
-        nd = sc.nodes;
-        tr = sc.tris;
-        return sc.meta->root;
+    using Index = uint32_t;
+    const float4* __restrict__ rays;
+    float4* __restrict__ hits;
+    const JobDev* jobs;
+    uint32_t n;
+    bool one_job;  // the job is known before the ray has arrived
+    float tmin, tmax;
+    __device__ __forceinline__ uint32_t load(uint32_t i, float4& r0, float4& r1, const void*& nd, const Tri*& tr) const {
+        r0 = __ldg(rays + 2ull * i);
+        r1 = __ldg(rays + 2ull * i + 1);
+        const uint32_t root = job_bvh<LAYOUT>(jobs, one_job ? 0u : __float_as_uint(r1.w), nd, tr);
+        r1.z = tmin;
+        r1.w = tmax;
+        return root;
     }
-    __device__ __forceinline__ void finish(uint64_t i, const trav::Lane& L) const {
-        const uint32_t pid = q[i];
-        ps->hit[pid] = L.best_prim == 0xFFFFFFFFu ? make_float4(L.p.tmax, __int_as_float(-1), 0.0f, 0.0f)
-                                                  : make_float4(L.best_t, __uint_as_float(L.best_prim), L.bu, L.bv);
+    template <class L>
+    __device__ __forceinline__ void finish(uint32_t i, const L& l) const {
+        hits[i] = l.best_prim == 0xFFFFFFFFu ? make_float4(l.p.tmax, __int_as_float(-1), 0.0f, 0.0f)
+                                             : make_float4(l.best_t, __uint_as_float(l.best_prim), l.bu, l.bv);
     }
 };
 
@@ -343,33 +359,40 @@ template <int LAYOUT, int SSTACK>
 __global__ void __launch_bounds__(trav::kMaxTraceThreads, 4) k_trace_queue(Paths ps, int b) {
     extern __shared__ int2 s_stack[];
     if (b > (int)ps.hdr->max_depth) return;
-    QueueSrc src{(b & 1) ? ps.qb : ps.qa, &ps, ps.cnt[b]};
+    QueueSrc<LAYOUT> src{(b & 1) ? ps.ray[1] : ps.ray[0], ps.hit, ps.jobs, ps.cnt[b], ps.hdr->njobs == 1,
+                         b == 0 ? kCameraTmin : kScatterTmin, b == 0 ? kCameraTmax : kScatterTmax};
     trav::traverse_loop<false, LAYOUT, SSTACK, trav::kRefillQueue>(src, ps.work + b, ps.cnt + kErrWord, s_stack);
 }
 
 // Shadow rays: an unoccluded ray adds its contribution to its path
 // (accumulate_light_sampling_contribution_kernel, pathtracer_kernel.h:642-664).
+template <int LAYOUT>
 struct ShadowSrc {
-    const Paths* ps;
-    uint64_t n;
-    __device__ __forceinline__ uint32_t load(uint64_t i, float4& r0, float4& r1, const void*& nd, const Tri*& tr) const {
-        r0 = ps->sray[2 * i];
-        r1 = ps->sray[2 * i + 1];
-        const uint32_t pid = __float_as_uint(ps->scon[i].w);
-        const SceneDev& sc = ps->jobs[ps->job[pid]].sc;
-        nd = sc.nodes;
-        tr = sc.tris;
-        return sc.meta->root;
+    using Index = uint32_t;
+    const float4* __restrict__ rays;
+    const float4* __restrict__ con;
+    float4* acc;
+    const JobDev* jobs;
+    uint32_t n;
+    bool one_job;
+    __device__ __forceinline__ uint32_t load(uint32_t i, float4& r0, float4& r1, const void*& nd, const Tri*& tr) const {
+        r0 = __ldg(rays + 2ull * i);
+        r1 = __ldg(rays + 2ull * i + 1);
+        const uint32_t root = job_bvh<LAYOUT>(jobs, one_job ? 0u : __float_as_uint(r1.z), nd, tr);
+        r1.z = kShadowTmin;
+        r1.w = kShadowTmax;
+        return root;
     }
-    __device__ __forceinline__ void finish(uint64_t i, const trav::Lane& L) const {
-        if (L.best_prim != 0xFFFFFFFFu) return;
-        const float4 c = ps->scon[i];
+    template <class L>
+    __device__ __forceinline__ void finish(uint32_t i, const L& l) const {
+        if (l.best_prim != 0xFFFFFFFFu) return;
+        const float4 c = __ldg(con + i);
         const uint32_t pid = __float_as_uint(c.w);
-        float4 a = ps->acc[pid];
+        float4 a = acc[pid];
         a.x += c.x;
         a.y += c.y;
         a.z += c.z;
-        ps->acc[pid] = a;
+        acc[pid] = a;
     }
 };
 
@@ -377,35 +400,39 @@ template <int LAYOUT, int SSTACK>
 __global__ void __launch_bounds__(trav::kMaxTraceThreads, 4) k_trace_shadow(Paths ps, int b) {
     extern __shared__ int2 s_stack[];
     if (b >= (int)ps.hdr->max_depth) return;
-    ShadowSrc src{&ps, ps.cnt[kShadowBase + b]};
+    ShadowSrc<LAYOUT> src{ps.sray, ps.scon, ps.acc, ps.jobs, ps.cnt[kShadowBase + b], ps.hdr->njobs == 1};
     trav::traverse_loop<true, LAYOUT, SSTACK, trav::kRefillQueue>(src, ps.work + kShadowBase + b, ps.cnt + kErrWord,
                                                                    s_stack);
 }
 
 // ---- shading groups -----------------------------------------------------------------
-// Regroups the paths of bounce b by what their ray hit (group 0: a miss; 1 + t:
-// a surface of material type t), appending each path id to its group with one
-// atomic per warp and group. The order inside a group is arbitrary; shading
+// Regroups the queue entries of bounce b by what their ray hit (group 0: a miss;
+// 1 + t: a surface of material type t), appending each entry to its group with
+// one atomic per warp and group. The order inside a group is arbitrary; shading
 // depends on nothing but the path's own state, so images do not change.
 // (Filing the paths in the closest-hit kernel's epilogue instead measured
 // slower: the extra gathers lengthened that kernel by as much as this one takes.)
+__device__ __forceinline__ uint32_t* bin_entry(const Paths& ps, int k, uint32_t at) {
+    uint32_t* a = ps.bins + (size_t)(k >> 1) * ps.capacity;
+    return (k & 1) ? a + (ps.capacity - 1 - at) : a + at;
+}
+
 __global__ void __launch_bounds__(kShadeThreads) k_bin(Paths ps, int b) {
     if (b > (int)ps.hdr->max_depth) return;
     const uint32_t n = ps.cnt[b];
-    const uint32_t* q = (b & 1) ? ps.qb : ps.qa;
+    const float4* rays = (b & 1) ? ps.ray[1] : ps.ray[0];
+    const bool one_job = ps.hdr->njobs == 1;
     uint32_t* cnt = ps.cnt + kBinBase + kShadeBins * b;
     const uint32_t stride = gridDim.x * blockDim.x;
     const int lane = threadIdx.x & 31;
     for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += stride) {
         const uint32_t i = base + threadIdx.x;
         int bin = -1;
-        uint32_t pid = 0;
         if (i < n) {
-            pid = q[i];
-            const int32_t prim = __float_as_int(ps.hit[pid].y);
+            const int32_t prim = __float_as_int(ps.hit[i].y);
             bin = 0;
             if (prim >= 0) {
-                const SceneDev& sc = ps.jobs[ps.job[pid]].sc;
+                const SceneDev& sc = ps.jobs[one_job ? 0u : __float_as_uint(rays[2ull * i + 1].w)].sc;
                 bin = 1 + min((int)sc.mats[sc.tri_mat[prim] & 0x3FFFFFFFu].type, kShadeBins - 2);
             }
         }
@@ -417,7 +444,7 @@ __global__ void __launch_bounds__(kShadeThreads) k_bin(Paths ps, int b) {
             uint32_t at = 0;
             if (lane == leader) at = atomicAdd(cnt + k, (uint32_t)__popc(m));
             at = __shfl_sync(0xFFFFFFFFu, at, leader);
-            if (bin == k) ps.bins[(size_t)k * ps.capacity + at + __popc(m & lane_lt())] = pid;
+            if (bin == k) *bin_entry(ps, k, at + __popc(m & lane_lt())) = i;
         }
     }
 }
@@ -434,7 +461,7 @@ __global__ void __launch_bounds__(kShadeThreads) k_bin(Paths ps, int b) {
 // BINNED: read the bounce's paths in k_bin's groups, as one array; else the
 // queue itself (waves whose scenes use one material type).
 template <bool BINNED>
-__global__ void __launch_bounds__(kShadeThreads, 4) k_shade(Paths ps, int b) {
+__global__ void __launch_bounds__(kShadeThreads, 4) k_shade(Paths ps, int b, PcgJump jump) {
     if (b > (int)ps.hdr->max_depth) return;
     __shared__ uint32_t s_first[kShadeBins + 1];
     if (BINNED) {
@@ -449,42 +476,50 @@ __global__ void __launch_bounds__(kShadeThreads, 4) k_shade(Paths ps, int b) {
         __syncthreads();
     }
     const uint32_t n = BINNED ? s_first[kShadeBins] : ps.cnt[b];
-    const uint32_t* q = (b & 1) ? ps.qb : ps.qa;
-    uint32_t* qn = (b & 1) ? ps.qa : ps.qb;
+    const float4* rays = (b & 1) ? ps.ray[1] : ps.ray[0];
+    const float4* thrs = (b & 1) ? ps.thr[1] : ps.thr[0];
+    float4* rays_next = (b & 1) ? ps.ray[0] : ps.ray[1];
+    float4* thrs_next = (b & 1) ? ps.thr[0] : ps.thr[1];
+    const bool one_job = ps.hdr->njobs == 1;
     const uint32_t stride = gridDim.x * blockDim.x;
     for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += stride) {
         const uint32_t i = base + threadIdx.x;
         bool scatter = false, shadow = false;
-        uint32_t pid = 0;
         float4 new_r0, new_r1, sh_r0, sh_r1, sh_c;
         float4 new_thr;
-        uint32_t new_flags = 0;
         if (i < n) {
+            uint32_t e = i;  // queue entry
             if (BINNED) {
                 int k = 0;
                 while (k + 1 < kShadeBins && i >= s_first[k + 1]) ++k;
-                pid = ps.bins[(size_t)k * ps.capacity + (i - s_first[k])];
-            } else {
-                pid = q[i];
+                e = *bin_entry(ps, k, i - s_first[k]);
             }
-            const JobDev& J = ps.jobs[ps.job[pid]];
+            const float4 r0 = rays[2ull * e], r1 = rays[2ull * e + 1];
+            const float4 hv = ps.hit[e];
+            const float4 th = b == 0 ? make_float4(1.0f, 1.0f, 1.0f, 0.0f) : thrs[e];
+            const uint32_t pid = __float_as_uint(r1.z);
+            const JobDev& J = ps.jobs[one_job ? 0u : __float_as_uint(r1.w)];
             const SceneDev& sc = J.sc;
             const bool compat = (J.flags & GR_RENDER_REFERENCE_COMPAT) != 0;
-            const uint32_t pixel = (pid - J.path_base) % J.npix;
+            const uint32_t local = pid - J.path_base;
+            const uint32_t pixel = local % J.npix;
             const uint64_t inc = pcg_inc(pixel);
-            uint64_t st = ps.rng[pid];
-            const float4 r0 = ps.ray[2ull * pid], r1 = ps.ray[2ull * pid + 1];
-            const float4 hv = ps.hit[pid];
-            float4 th = ps.thr[pid];
-            const uint32_t flags = ps.flags[pid];
+            uint64_t st = pcg_seed(J.seed + (uint64_t)(J.sample_base + local / J.npix) * kSampleStride, inc);
+            st = st * jump.mul + inc * jump.add;
+            const bool specular = (__float_as_uint(th.w) & kSpecularBit) != 0;
             V3 thr = v3(th.x, th.y, th.z);
+            V3 L0 = vs(0.0f);  // bounce 0 writes the path's radiance, later bounces add to it
+            auto add = [&](V3 L) {
+                if (b == 0) L0 = L0 + L;
+                else add_acc(ps, pid, L);
+            };
             const V3 rd = v3(r0.w, r1.x, r1.y);
             const int32_t prim = __float_as_int(hv.y);
             bool alive = b <= (int)J.max_depth;
             bool as_miss = false;
             if (alive && b > 0) {
                 const float rr = pcg_float(st, inc);
-                if (prim >= 0 && !(flags & kFlagSpecular)) {
+                if (prim >= 0 && !specular) {
                     const DevMaterial* lm = sc.mats + (sc.tri_mat[prim] & 0x3FFFFFFFu);
                     if (lm->emissive) {
                         const Surf ls = surface(sc, (uint32_t)prim, hv.z, hv.w);
@@ -493,7 +528,7 @@ __global__ void __launch_bounds__(kShadeThreads, 4) k_shade(Paths ps, int b) {
                         const V3 Le = dot(-rd, ls.ns) > 0.0f ? v3(lm->er, lm->eg, lm->eb) : vs(0.0f);
                         const float bp = th.w;
                         const float w = (bp * bp) / (bp * bp + lpdf * lpdf);
-                        add_acc(ps, pid, thr * Le * w);
+                        add(thr * Le * w);
                     }
                 }
                 if (J.rr_depth >= 0 && (int)(b - 1) > J.rr_depth && maxc(thr) < 1.0f) {
@@ -510,14 +545,14 @@ __global__ void __launch_bounds__(kShadeThreads, 4) k_shade(Paths ps, int b) {
 #pragma unroll
                 for (int k = 0; k < 8; ++k) s[k] = pcg_float(st, inc);
                 if (prim < 0 || as_miss) {
-                    if (sc.has_env) add_acc(ps, pid, thr * env_radiance(sc, v3(r0.x, r0.y, r0.z), rd));
+                    if (sc.has_env) add(thr * env_radiance(sc, v3(r0.x, r0.y, r0.z), rd));
                 } else {
                     const uint32_t tm = sc.tri_mat[prim];
                     const DevMaterial* m = sc.mats + (tm & 0x3FFFFFFFu);
                     const Surf sf = surface(sc, (uint32_t)prim, hv.z, hv.w);
                     const V3 wo = -normalize(rd);
-                    if ((b == 0 || (flags & kFlagSpecular)) && m->emissive && dot(wo, sf.ns) > 0.0f)
-                        add_acc(ps, pid, thr * v3(m->er, m->eg, m->eb));
+                    if ((b == 0 || specular) && m->emissive && dot(wo, sf.ns) > 0.0f)
+                        add(thr * v3(m->er, m->eg, m->eb));
                     Bsdf bs;
                     bs.fr = make_frame(sf.ns);
                     bs.m = m;
@@ -546,7 +581,7 @@ __global__ void __launch_bounds__(kShadeThreads, 4) k_shade(Paths ps, int b) {
                                 const V3 so = sf.p - rd * 1.0e-4f;
                                 const V3 sd = ls.p - so;
                                 sh_r0 = make_float4(so.x, so.y, so.z, sd.x);
-                                sh_r1 = make_float4(sd.y, sd.z, 0.0f, 0.9999f);
+                                sh_r1 = make_float4(sd.y, sd.z, r1.w, 0.0f);
                                 sh_c = make_float4(c.x, c.y, c.z, __uint_as_float(pid));
                                 shadow = true;
                             }
@@ -557,14 +592,15 @@ __global__ void __launch_bounds__(kShadeThreads, 4) k_shade(Paths ps, int b) {
                     const V3 wgt = smp.pdf == 0.0f ? vs(0.0f) : thr * smp.f / smp.pdf;
                     if (!black(wgt)) {
                         new_r0 = make_float4(sf.p.x, sf.p.y, sf.p.z, smp.wi.x);
-                        new_r1 = make_float4(smp.wi.y, smp.wi.z, 1e-4f, 1e38f);
-                        new_thr = make_float4(wgt.x, wgt.y, wgt.z, smp.pdf);
-                        new_flags = smp.specular ? kFlagSpecular : 0u;
+                        new_r1 = make_float4(smp.wi.y, smp.wi.z, r1.z, r1.w);
+                        new_thr = make_float4(wgt.x, wgt.y, wgt.z,
+                                              __uint_as_float(__float_as_uint(fabsf(smp.pdf)) |
+                                                              (smp.specular ? kSpecularBit : 0u)));
                         scatter = true;
                     }
                 }
             }
-            ps.rng[pid] = st;
+            if (b == 0) ps.acc[pid] = make_float4(L0.x, L0.y, L0.z, 0.0f);
         }
         const uint32_t sslot = warp_append(ps.cnt + kShadowBase + b, shadow);
         const uint32_t nslot = warp_append(ps.cnt + b + 1, scatter);
@@ -574,11 +610,9 @@ __global__ void __launch_bounds__(kShadeThreads, 4) k_shade(Paths ps, int b) {
             ps.scon[sslot] = sh_c;
         }
         if (scatter) {
-            ps.ray[2ull * pid] = new_r0;
-            ps.ray[2ull * pid + 1] = new_r1;
-            ps.thr[pid] = new_thr;
-            ps.flags[pid] = new_flags;
-            qn[nslot] = pid;
+            rays_next[2ull * nslot] = new_r0;
+            rays_next[2ull * nslot + 1] = new_r1;
+            thrs_next[nslot] = new_thr;
         }
     }
 }
@@ -670,11 +704,12 @@ cudaError_t issue_wave_l(const Paths& ps, uint32_t depth_steps, int tgrid, int t
     k_camera<<<sgrid, kShadeThreads, 0, s>>>(ps);
     for (int b = 0; b <= (int)depth_steps; ++b) {
         k_trace_queue<LAYOUT, SSTACK><<<tgrid, tblock, smem, s>>>(ps, b);
+        const PcgJump jump = pcg_jump(draws_before(b));
         if (bin) {
             k_bin<<<sgrid, kShadeThreads, 0, s>>>(ps, b);
-            k_shade<true><<<sgrid, kShadeThreads, 0, s>>>(ps, b);
+            k_shade<true><<<sgrid, kShadeThreads, 0, s>>>(ps, b, jump);
         } else {
-            k_shade<false><<<sgrid, kShadeThreads, 0, s>>>(ps, b);
+            k_shade<false><<<sgrid, kShadeThreads, 0, s>>>(ps, b, jump);
         }
         if (b < (int)depth_steps) k_trace_shadow<LAYOUT, SSTACK><<<tgrid, tblock, smem, s>>>(ps, b);
     }
@@ -733,16 +768,11 @@ size_t path_layout(uint32_t cap, char* base, Paths* ps) {
         return p;
     };
     const size_t c = cap;
-    ps->ray = (float4*)take(32 * c);
+    for (int k = 0; k < 2; ++k) ps->ray[k] = (float4*)take(32 * c);
+    for (int k = 0; k < 2; ++k) ps->thr[k] = (float4*)take(16 * c);
     ps->hit = (float4*)take(16 * c);
-    ps->thr = (float4*)take(16 * c);
     ps->acc = (float4*)take(16 * c);
-    ps->flags = (uint32_t*)take(4 * c);
-    ps->job = (uint32_t*)take(4 * c);
-    ps->rng = (unsigned long long*)take(8 * c);
-    ps->qa = (uint32_t*)take(4 * c);
-    ps->qb = (uint32_t*)take(4 * c);
-    ps->bins = (uint32_t*)take(4 * kShadeBins * c);
+    ps->bins = (uint32_t*)take(4 * ((kShadeBins + 1) / 2) * c);
     ps->sray = (float4*)take(32 * c);
     ps->scon = (float4*)take(16 * c);
     ps->cnt = (uint32_t*)take(sizeof(uint32_t) * kCntWords);
@@ -903,7 +933,7 @@ cudaError_t run_wave(WavePool& pool, const JobDev* h_jobs, uint32_t njobs, uint3
     const bool bin = __builtin_popcount(types) >= 2;
     if (!use_graph) return issue_wave(ps, max_depth, tgrid, sgrid, bin, s, tune);
     uint64_t key = 0x51ED270B27A3C1F5ull;
-    const uint64_t words[] = {(uint64_t)(uintptr_t)ps.ray, ps.capacity, steps, (uint64_t)tgrid, (uint64_t)sgrid,
+    const uint64_t words[] = {(uint64_t)(uintptr_t)ps.ray[0], ps.capacity, steps, (uint64_t)tgrid, (uint64_t)sgrid,
                               (uint64_t)tune.layout, (uint64_t)tune.block, (uint64_t)tune.sstack, (uint64_t)bin};
     for (uint64_t w : words) key = mix64(key, w);
     int hit = -1;

@@ -97,20 +97,30 @@ struct WaveHeader {
     unsigned long long closest_rays, shadow_rays;  // running totals
 };
 
-// Path state for one wave, indexed by path id.
+// Path state for one wave. What the next bounce needs of a path (its ray and
+// throughput) lives at the path's place in the bounce's queue, not at its path
+// id: queues are appended to and read front to back, so tracing and shading
+// stream whole sectors, where state kept at the path id was visited in queue
+// order, strewn over memory (a 16-byte record then costs its 32- or 64-byte
+// fetch). Two buffers alternate by bounce. The RNG state is not stored: a path
+// that is alive has drawn the same count of numbers as every other path of its
+// bounce, so the state follows from (seed, pixel, sample) by one jump. Bytes
+// per path: 64 + 32 + 16 + 16 + 12 + 32 + 16 = 188.
 struct Paths {
-    float4* ray;    // 2 per path: (o.xyz, d.x), (d.y, d.z, tmin, tmax)
-    float4* hit;    // (t, prim bits, u, v)
-    float4* thr;    // (throughput rgb, pdf of the last BSDF sample)
-    float4* acc;    // (radiance rgb, 0)
-    uint32_t* flags;
-    uint32_t* job;  // job of each path
-    unsigned long long* rng;
-    uint32_t* qa;   // path-id queues, ping-pong by bounce
-    uint32_t* qb;
-    uint32_t* bins; // the bounce's queue regrouped for shading: kShadeBins runs of capacity entries
-    float4* sray;   // shadow rays, 2 per entry
-    float4* scon;   // shadow contribution (rgb, pid bits)
+    // 2 per queue entry: (o.xyz, d.x), (d.y, d.z, path id bits, job bits); the
+    // interval is a bounce's constant (camera rays 0 .. 1e34, scattered rays
+    // 1e-4 .. 1e38). Bounce b reads buffer b & 1 and its shading writes the other.
+    float4* ray[2];
+    // per queue entry (unused in bounce 0, where it is 1): throughput rgb, and
+    // the pdf of the last BSDF sample with the sign bit set after a specular bounce
+    float4* thr[2];
+    float4* hit;    // per queue entry: (t, prim bits, u, v)
+    float4* acc;    // per path id: (radiance rgb, 0)
+    // the bounce's queue entries grouped for shading: group k in array k / 2,
+    // from its front when k is even, from its back when k is odd
+    uint32_t* bins;
+    float4* sray;   // shadow rays, 2 per entry: (o.xyz, d.x), (d.y, d.z, job bits, 0); interval 0 .. 0.9999
+    float4* scon;   // shadow contribution (rgb, path id bits)
     uint32_t* cnt;  // [0, kMaxDepth]: closest queue sizes; [kMaxDepth+1, ...]: shadow queue sizes
     unsigned long long* work;  // dynamic-fetch counters, one per trace launch of a wave
     WaveHeader* hdr;

@@ -57,6 +57,19 @@ __device__ __forceinline__ uint64_t pcg_seed(uint64_t initstate, uint64_t inc) {
     pcg_next(st, inc);
     return st;
 }
+// The state after k further draws is mul * state + add * inc (k steps of the
+// LCG composed: mul = a^k, add = 1 + a + ... + a^(k-1)).
+struct PcgJump {
+    uint64_t mul, add;
+};
+inline PcgJump pcg_jump(uint32_t k) {
+    PcgJump j{1ull, 0ull};
+    for (; k; --k) {
+        j.add = j.add * 6364136223846793005ull + 1ull;
+        j.mul *= 6364136223846793005ull;
+    }
+    return j;
+}
 // 24-bit uniform float in [0, 1)
 __device__ __forceinline__ float pcg_float(uint64_t& state, uint64_t inc) {
     return (float)(pcg_next(state, inc) >> 8) * 0x1p-24f;

@@ -134,21 +134,22 @@ __device__ __forceinline__ uint32_t lanemask_lt() {
 // Per-lane traversal state. A lane owns one ray at a time; when its ray
 // finishes the lane goes idle and is refilled with a new ray once enough lanes
 // of the warp are idle, so long-tailed rays do not hold a whole warp.
+template <class Index>
 struct Lane {
     const void* nodes;  // BVH of this lane's ray (rays of one queue may belong to different scenes)
     const Tri* tris;
     RayW p;
     float best_t, bu, bv;
     uint32_t best_prim;
-    uint64_t ray;
+    Index ray;
     int32_t node;
     int sp;
 };
 
 // Tests leaf triangle `c` (~sorted position); returns true when an any-hit
 // query is answered. Closest-hit ties at equal t go to the smaller prim id.
-template <bool ANY>
-__device__ __forceinline__ bool leaf(Lane& L, int32_t c) {
+template <bool ANY, class L_>
+__device__ __forceinline__ bool leaf(L_& L, int32_t c) {
     const Tri* tr = L.tris + (uint32_t)(~c);
     const float4 a = __ldg(&tr->a), b = __ldg(&tr->b), cc = __ldg(&tr->c);
     float t, u, v;
@@ -167,8 +168,8 @@ __device__ __forceinline__ bool leaf(Lane& L, int32_t c) {
 // Pushes a deferred node with its entry distance; false on overflow. The
 // first SSTACK entries of a thread live in shared memory ([entry][thread],
 // conflict-free), deeper entries in a local array.
-template <int SSTACK>
-__device__ __forceinline__ bool push(Lane& L, int32_t c, float tn, int2* s_stack, int2* l_stack, uint32_t* err) {
+template <int SSTACK, class L_>
+__device__ __forceinline__ bool push(L_& L, int32_t c, float tn, int2* s_stack, int2* l_stack, uint32_t* err) {
     if (L.sp < SSTACK) {
         s_stack[L.sp * blockDim.x + threadIdx.x] = make_int2(c, __float_as_int(tn));
     } else if (L.sp < kStackMax) {
@@ -183,8 +184,8 @@ __device__ __forceinline__ bool push(Lane& L, int32_t c, float tn, int2* s_stack
 
 // Pops the next deferred node still in front of the closest hit; false when
 // the stack is empty (the ray is finished).
-template <bool ANY, int SSTACK>
-__device__ __forceinline__ bool pop(Lane& L, const int2* s_stack, const int2* l_stack, int32_t& next) {
+template <bool ANY, int SSTACK, class L_>
+__device__ __forceinline__ bool pop(L_& L, const int2* s_stack, const int2* l_stack, int32_t& next) {
     for (;;) {
         if (L.sp == 0) return false;
         --L.sp;
@@ -198,8 +199,8 @@ __device__ __forceinline__ bool pop(Lane& L, const int2* s_stack, const int2* l_
 
 // One binary node: both child boxes, nearer first; leaves tested inline.
 // Returns true when the ray is finished.
-template <bool ANY, int SSTACK>
-__device__ __forceinline__ bool trace_step2(Lane& L, int2* s_stack, int2* l_stack, uint32_t* err) {
+template <bool ANY, int SSTACK, class L_>
+__device__ __forceinline__ bool trace_step2(L_& L, int2* s_stack, int2* l_stack, uint32_t* err) {
     const float4* q = reinterpret_cast<const float4*>(static_cast<const Node*>(L.nodes) + L.node);
     float4 q0, q1, q2, q3f;
     ldg32B(q, q0, q1);
@@ -242,8 +243,8 @@ __device__ __forceinline__ float qplane(uint32_t word, int k, float scale, float
 // visited in order of (entry distance, slot); leaves tested inline, the nearest
 // inner child visited next, the other inner children pushed so the nearer pop
 // first. Returns true when the ray is finished.
-template <bool ANY, bool QUANT, int SSTACK>
-__device__ __forceinline__ bool trace_step4(Lane& L, int2* s_stack, int2* l_stack, uint32_t* err) {
+template <bool ANY, bool QUANT, int SSTACK, class L_>
+__device__ __forceinline__ bool trace_step4(L_& L, int2* s_stack, int2* l_stack, uint32_t* err) {
     float tn[4];
     bool h[4];
     int32_t c[4];
@@ -453,8 +454,8 @@ __device__ __forceinline__ void stack_put(int i, int2 v, int2* s_stack, int2* l_
 }
 
 // Leaf triangle `idx` of the layout's own triangle array.
-template <bool ANY>
-__device__ __forceinline__ bool leaf_at(Lane& L, uint32_t idx) { return leaf<ANY>(L, ~(int32_t)idx); }
+template <bool ANY, class L_>
+__device__ __forceinline__ bool leaf_at(L_& L, uint32_t idx) { return leaf<ANY>(L, ~(int32_t)idx); }
 
 // One 8-wide node. A child plane is q * 2^e + lo, taken exactly; its ray
 // distance q * S + C, with S = 2^e / d (exact: a power-of-two scaling) and
@@ -467,8 +468,8 @@ __device__ __forceinline__ bool leaf_at(Lane& L, uint32_t idx) { return leaf<ANY
 // slot ^ octant and the lowest rank is visited next. The remaining inner hits
 // stay on the stack as one group entry (child_base, inner mask | hits << 8),
 // taken one child at a time. Returns true when the ray is finished.
-template <bool ANY, int SSTACK>
-__device__ __forceinline__ bool trace_step8(Lane& L, int2* s_stack, int2* l_stack, uint32_t* err,
+template <bool ANY, int SSTACK, class L_>
+__device__ __forceinline__ bool trace_step8(L_& L, int2* s_stack, int2* l_stack, uint32_t* err,
                                             const unsigned char* perm8) {
     const float4* q = reinterpret_cast<const float4*>(static_cast<const Node8Q*>(L.nodes) + L.node);
     float4 h0, h1, b0, b1, c0, c1;
@@ -559,8 +560,8 @@ __device__ __forceinline__ bool trace_step8(Lane& L, int2* s_stack, int2* l_stac
     return last;
 }
 
-template <bool ANY, int LAYOUT, int SSTACK>
-__device__ __forceinline__ bool trace_step(Lane& L, int2* s_stack, int2* l_stack, uint32_t* err,
+template <bool ANY, int LAYOUT, int SSTACK, class L_>
+__device__ __forceinline__ bool trace_step(L_& L, int2* s_stack, int2* l_stack, uint32_t* err,
                                            const unsigned char* perm8) {
     if (LAYOUT == kLayoutBvh2) return trace_step2<ANY, SSTACK>(L, s_stack, l_stack, err);
     if (LAYOUT == kLayoutBvh8Q8) return trace_step8<ANY, SSTACK>(L, s_stack, l_stack, err, perm8);
@@ -569,20 +570,21 @@ __device__ __forceinline__ bool trace_step(Lane& L, int2* s_stack, int2* l_stack
 
 // A warp refills its idle lanes once at least REFILL of them are idle. The
 // ray-query kernels use 4 (a ray loads in two 16-byte reads; 2, 6 and 8
-// measured slower); the render's queue kernels use 12 (a queued path also looks
-// up its job and scene; 4, 6, 8, 16 and 20 measured slower on the Cornell and
-// glossy renders).
+// measured slower); the render's queue kernels use 12 (a queued ray also looks
+// up its job and scene; glossy 1024 x 768 x 64 spp: 72.4 ms at 8 and 12, 74.5 at
+// 4, 74.1 at 16).
 constexpr int kRefillRays = 4;
 constexpr int kRefillQueue = 12;
 
 // Persistent dynamic-fetch loop. `Src` supplies the work:
-//   uint64_t n                                        number of rays
-//   uint32_t load(uint64_t i, float4& r0, float4& r1, const void*& nodes,
+//   Index                                             integer type of a ray's index
+//   n                                                 number of rays
+//   uint32_t load(Index i, float4& r0, float4& r1, const void*& nodes,
 //                 const Tri*& tris)                   ray i (reference Ray layout) and
 //                                                     its BVH (nodes and triangles of
 //                                                     layout LAYOUT); returns the binary
 //                                                     root (kNoNode when empty)
-//   void finish(uint64_t i, const Lane& L)            ray i is done (L.best_prim ==
+//   void finish(Index i, const Lane<Index>& L)        ray i is done (L.best_prim ==
 //                                                     0xFFFFFFFF means a miss)
 // The shared stack has SSTACK x blockDim.x int2 entries (dynamic shared memory),
 // followed for the 8-wide layout by the octant permutation table
@@ -600,8 +602,9 @@ __device__ __forceinline__ void traverse_loop(Src& src, unsigned long long* coun
     }
     const int lane = threadIdx.x & 31;
     const uint32_t ltmask = lanemask_lt();
+    using Index = typename Src::Index;
     const uint64_t n = src.n;
-    Lane L;
+    Lane<Index> L;
     bool active = false;
     bool exhausted = false;
     for (;;) {
@@ -618,18 +621,18 @@ __device__ __forceinline__ void traverse_loop(Src& src, unsigned long long* coun
                 const uint64_t i = base + __popc(idle & ltmask);
                 if (i < n) {
                     float4 r0, r1;
-                    const uint32_t root = src.load(i, r0, r1, L.nodes, L.tris);
+                    const uint32_t root = src.load((Index)i, r0, r1, L.nodes, L.tris);
                     L.p = prepare(r0, r1);
                     L.best_t = L.p.tmax;
                     L.bu = 0.0f;
                     L.bv = 0.0f;
                     L.best_prim = 0xFFFFFFFFu;
-                    L.ray = i;
+                    L.ray = (Index)i;
                     L.node = (LAYOUT == kLayoutBvh8Q8 && root != kNoNode) ? 0 : (int32_t)root;  // 8-wide root is node 0
                     L.sp = 0;
                     active = true;
                     if (root == kNoNode) {
-                        src.finish(i, L);
+                        src.finish((Index)i, L);
                         active = false;
                     }
                 }
