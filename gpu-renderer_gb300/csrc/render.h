@@ -120,7 +120,7 @@ struct Paths {
     // the bounce's queue entries grouped for shading: group k in array k / 2,
     // from its front when k is even, from its back when k is odd
     uint32_t* bins;
-    float4* sray;   // shadow rays, 2 per entry: (o.xyz, d.x), (d.y, d.z, job bits, 0); interval 0 .. 0.9999
+    float4* sray;   // shadow rays, 2 per entry: (o.xyz, d.x), (d.y, d.z, 0, job bits); interval 0 .. 0.9999
     float4* scon;   // shadow contribution (rgb, path id bits)
     uint32_t* cnt;  // [0, kMaxDepth]: closest queue sizes; [kMaxDepth+1, ...]: shadow queue sizes
     unsigned long long* work;  // dynamic-fetch counters, one per trace launch of a wave

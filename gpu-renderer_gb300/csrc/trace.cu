@@ -52,7 +52,7 @@ __global__ void __launch_bounds__(trav::kMaxTraceThreads, 4) k_trace(const void*
                                                                   uint32_t* err) {
     extern __shared__ int2 s_stack[];
     RaySrc src{rays, hits, n, nodes, tris, meta->root};
-    trav::traverse_loop<ANY, LAYOUT, SSTACK, trav::kRefillRays>(src, counter, err, s_stack);
+    trav::traverse_loop<ANY ? trav::kAny : trav::kClosest, LAYOUT, SSTACK, trav::kRefillRays>(src, counter, err, s_stack);
 }
 
 template <bool ANY, int LAYOUT, int SSTACK>

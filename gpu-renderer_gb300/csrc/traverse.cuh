@@ -142,27 +142,34 @@ struct Lane {
     float best_t, bu, bv;
     uint32_t best_prim;
     Index ray;
+    bool any;  // kMixed: this ray ends at its first hit
     int32_t node;
     int sp;
 };
 
+// What a kernel's rays ask for: all the closest hit, all any hit, or each its
+// own (Lane::any).
+enum Query : int { kClosest = 0, kAny = 1, kMixed = 2 };
+
+template <int Q, class L_>
+__device__ __forceinline__ bool wants_any(const L_& L) {
+    return Q == kMixed ? L.any : Q == kAny;
+}
+
 // Tests leaf triangle `c` (~sorted position); returns true when an any-hit
 // query is answered. Closest-hit ties at equal t go to the smaller prim id.
-template <bool ANY, class L_>
+template <int Q, class L_>
 __device__ __forceinline__ bool leaf(L_& L, int32_t c) {
     const Tri* tr = L.tris + (uint32_t)(~c);
     const float4 a = __ldg(&tr->a), b = __ldg(&tr->b), cc = __ldg(&tr->c);
     float t, u, v;
     if (!tri_test(L.p, a, b, cc, L.best_t, t, u, v)) return false;
     const uint32_t prim = __float_as_uint(a.w);
-    if (ANY) {
-        L.best_t = t; L.bu = u; L.bv = v; L.best_prim = prim;
-        return true;
-    }
-    if (t < L.best_t || prim < L.best_prim) {
+    const bool any = wants_any<Q>(L);
+    if (any || t < L.best_t || prim < L.best_prim) {
         L.best_t = t; L.bu = u; L.bv = v; L.best_prim = prim;
     }
-    return false;
+    return any;
 }
 
 // Pushes a deferred node with its entry distance; false on overflow. The
@@ -184,13 +191,13 @@ __device__ __forceinline__ bool push(L_& L, int32_t c, float tn, int2* s_stack, 
 
 // Pops the next deferred node still in front of the closest hit; false when
 // the stack is empty (the ray is finished).
-template <bool ANY, int SSTACK, class L_>
+template <int Q, int SSTACK, class L_>
 __device__ __forceinline__ bool pop(L_& L, const int2* s_stack, const int2* l_stack, int32_t& next) {
     for (;;) {
         if (L.sp == 0) return false;
         --L.sp;
         const int2 e = L.sp < SSTACK ? s_stack[L.sp * blockDim.x + threadIdx.x] : l_stack[L.sp - SSTACK];
-        if (ANY || __int_as_float(e.y) <= __fmul_rn(L.best_t, kCullSlack)) {
+        if (Q == kAny || __int_as_float(e.y) <= __fmul_rn(L.best_t, kCullSlack)) {
             next = e.x;
             return true;
         }
@@ -199,7 +206,7 @@ __device__ __forceinline__ bool pop(L_& L, const int2* s_stack, const int2* l_st
 
 // One binary node: both child boxes, nearer first; leaves tested inline.
 // Returns true when the ray is finished.
-template <bool ANY, int SSTACK, class L_>
+template <int Q, int SSTACK, class L_>
 __device__ __forceinline__ bool trace_step2(L_& L, int2* s_stack, int2* l_stack, uint32_t* err) {
     const float4* q = reinterpret_cast<const float4*>(static_cast<const Node*>(L.nodes) + L.node);
     float4 q0, q1, q2, q3f;
@@ -221,7 +228,7 @@ __device__ __forceinline__ bool trace_step2(L_& L, int2* s_stack, int2* l_stack,
         const int32_t c = s == 0 ? cn : cf;
         if (!h) continue;
         if (c < 0) {
-            if (leaf<ANY>(L, c)) return true;
+            if (leaf<Q>(L, c)) return true;
         } else if (!have) {
             next = c;
             have = true;
@@ -229,7 +236,7 @@ __device__ __forceinline__ bool trace_step2(L_& L, int2* s_stack, int2* l_stack,
             return true;
         }
     }
-    if (!have && !pop<ANY, SSTACK>(L, s_stack, l_stack, next)) return true;
+    if (!have && !pop<Q, SSTACK>(L, s_stack, l_stack, next)) return true;
     L.node = next;
     return false;
 }
@@ -243,7 +250,7 @@ __device__ __forceinline__ float qplane(uint32_t word, int k, float scale, float
 // visited in order of (entry distance, slot); leaves tested inline, the nearest
 // inner child visited next, the other inner children pushed so the nearer pop
 // first. Returns true when the ray is finished.
-template <bool ANY, bool QUANT, int SSTACK, class L_>
+template <int Q, bool QUANT, int SSTACK, class L_>
 __device__ __forceinline__ bool trace_step4(L_& L, int2* s_stack, int2* l_stack, uint32_t* err) {
     float tn[4];
     bool h[4];
@@ -318,7 +325,7 @@ __device__ __forceinline__ bool trace_step4(L_& L, int2* s_stack, int2* l_stack,
             }
         if (!hr) continue;
         if (cr < 0) {
-            if (leaf<ANY>(L, cr)) return true;
+            if (leaf<Q>(L, cr)) return true;
         } else if (!have) {
             next = cr;
             have = true;
@@ -332,7 +339,7 @@ __device__ __forceinline__ bool trace_step4(L_& L, int2* s_stack, int2* l_stack,
     if (np > 2 && !push<SSTACK>(L, pc2, pt2, s_stack, l_stack, err)) return true;
     if (np > 1 && !push<SSTACK>(L, pc1, pt1, s_stack, l_stack, err)) return true;
     if (np > 0 && !push<SSTACK>(L, pc0, pt0, s_stack, l_stack, err)) return true;
-    if (!have && !pop<ANY, SSTACK>(L, s_stack, l_stack, next)) return true;
+    if (!have && !pop<Q, SSTACK>(L, s_stack, l_stack, next)) return true;
     L.node = next;
     return false;
 }
@@ -454,8 +461,8 @@ __device__ __forceinline__ void stack_put(int i, int2 v, int2* s_stack, int2* l_
 }
 
 // Leaf triangle `idx` of the layout's own triangle array.
-template <bool ANY, class L_>
-__device__ __forceinline__ bool leaf_at(L_& L, uint32_t idx) { return leaf<ANY>(L, ~(int32_t)idx); }
+template <int Q, class L_>
+__device__ __forceinline__ bool leaf_at(L_& L, uint32_t idx) { return leaf<Q>(L, ~(int32_t)idx); }
 
 // One 8-wide node. A child plane is q * 2^e + lo, taken exactly; its ray
 // distance q * S + C, with S = 2^e / d (exact: a power-of-two scaling) and
@@ -468,7 +475,7 @@ __device__ __forceinline__ bool leaf_at(L_& L, uint32_t idx) { return leaf<ANY>(
 // slot ^ octant and the lowest rank is visited next. The remaining inner hits
 // stay on the stack as one group entry (child_base, inner mask | hits << 8),
 // taken one child at a time. Returns true when the ray is finished.
-template <bool ANY, int SSTACK, class L_>
+template <int Q, int SSTACK, class L_>
 __device__ __forceinline__ bool trace_step8(L_& L, int2* s_stack, int2* l_stack, uint32_t* err,
                                             const unsigned char* perm8) {
     const float4* q = reinterpret_cast<const float4*>(static_cast<const Node8Q*>(L.nodes) + L.node);
@@ -554,18 +561,18 @@ __device__ __forceinline__ bool trace_step8(L_& L, int2* s_stack, int2* l_stack,
         do {
             const int k = __ffs(thits) - 1;
             thits &= thits - 1u;
-            if (leaf_at<ANY>(L, tri_base + __popc(leafmask & ((1u << k) - 1u)))) return true;
+            if (leaf_at<Q>(L, tri_base + __popc(leafmask & ((1u << k) - 1u)))) return true;
         } while (thits);
     }
     return last;
 }
 
-template <bool ANY, int LAYOUT, int SSTACK, class L_>
+template <int Q, int LAYOUT, int SSTACK, class L_>
 __device__ __forceinline__ bool trace_step(L_& L, int2* s_stack, int2* l_stack, uint32_t* err,
                                            const unsigned char* perm8) {
-    if (LAYOUT == kLayoutBvh2) return trace_step2<ANY, SSTACK>(L, s_stack, l_stack, err);
-    if (LAYOUT == kLayoutBvh8Q8) return trace_step8<ANY, SSTACK>(L, s_stack, l_stack, err, perm8);
-    return trace_step4<ANY, LAYOUT == kLayoutBvh4Q8, SSTACK>(L, s_stack, l_stack, err);
+    if (LAYOUT == kLayoutBvh2) return trace_step2<Q, SSTACK>(L, s_stack, l_stack, err);
+    if (LAYOUT == kLayoutBvh8Q8) return trace_step8<Q, SSTACK>(L, s_stack, l_stack, err, perm8);
+    return trace_step4<Q, LAYOUT == kLayoutBvh4Q8, SSTACK>(L, s_stack, l_stack, err);
 }
 
 // A warp refills its idle lanes once at least REFILL of them are idle. The
@@ -584,13 +591,14 @@ constexpr int kRefillQueue = 12;
 //                                                     its BVH (nodes and triangles of
 //                                                     layout LAYOUT); returns the binary
 //                                                     root (kNoNode when empty)
+//   bool any(Index i)                                 whether ray i asks for any hit (kMixed)
 //   void finish(Index i, const Lane<Index>& L)        ray i is done (L.best_prim ==
 //                                                     0xFFFFFFFF means a miss)
 // The shared stack has SSTACK x blockDim.x int2 entries (dynamic shared memory),
 // followed for the 8-wide layout by the octant permutation table
 // (traverse_smem). Every thread of the block calls it (the table is filled
 // behind a block barrier).
-template <bool ANY, int LAYOUT, int SSTACK, int REFILL, class Src>
+template <int Q, int LAYOUT, int SSTACK, int REFILL, class Src>
 __device__ __forceinline__ void traverse_loop(Src& src, unsigned long long* counter, uint32_t* err, int2* s_stack) {
     int2 l_stack[kStackMax - SSTACK];
     // 8-wide layout: xor_permute8 as a table (octant x mask, 2 KB after the
@@ -628,6 +636,7 @@ __device__ __forceinline__ void traverse_loop(Src& src, unsigned long long* coun
                     L.bv = 0.0f;
                     L.best_prim = 0xFFFFFFFFu;
                     L.ray = (Index)i;
+                    if constexpr (Q == kMixed) L.any = src.any((Index)i);
                     L.node = (LAYOUT == kLayoutBvh8Q8 && root != kNoNode) ? 0 : (int32_t)root;  // 8-wide root is node 0
                     L.sp = 0;
                     active = true;
@@ -638,7 +647,7 @@ __device__ __forceinline__ void traverse_loop(Src& src, unsigned long long* coun
                 }
             }
         }
-        if (active && trace_step<ANY, LAYOUT, SSTACK>(L, s_stack, l_stack, err, perm8)) {
+        if (active && trace_step<Q, LAYOUT, SSTACK>(L, s_stack, l_stack, err, perm8)) {
             src.finish(L.ray, L);
             active = false;
         }
