@@ -29,6 +29,35 @@ void DevBuf::release() {
     bytes = 0;
 }
 
+cudaError_t HostBuf::ensure(size_t want) {
+    cudaError_t e = cudaSuccess;
+    if (!done && (e = cudaEventCreateWithFlags(&done, cudaEventDisableTiming)) != cudaSuccess) {
+        done = nullptr;
+        return e;
+    }
+    if (want <= bytes && p) return cudaSuccess;
+    if (p) {  // its last use may still be in flight
+        cudaEventSynchronize(done);
+        cudaFreeHost(p);
+        p = nullptr;
+        bytes = 0;
+    }
+    if ((e = cudaMallocHost(&p, want ? want : 256)) != cudaSuccess) {
+        p = nullptr;
+        return e;
+    }
+    bytes = want;
+    return cudaSuccess;
+}
+
+void HostBuf::release() {
+    if (p) cudaFreeHost(p);
+    if (done) cudaEventDestroy(done);
+    p = nullptr;
+    done = nullptr;
+    bytes = 0;
+}
+
 void context_free(gr_ctx* ctx) {
     cudaSetDevice(ctx->device);
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
@@ -38,6 +67,7 @@ void context_free(gr_ctx* ctx) {
     ctx->scratch8.release();
     ctx->stage_in.release();
     ctx->stage_out.release();
+    for (HostBuf& b : ctx->image) b.release();
     if (ctx->stream2) cudaStreamSynchronize(ctx->stream2);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
     if (ctx->stream2) cudaStreamDestroy(ctx->stream2);

@@ -122,6 +122,20 @@ struct DevBuf {
     ~DevBuf() { release(); }
 };
 
+// Page-locked host buffer owned by an object, with an event for its last use;
+// grows on demand, never shrinks.
+struct HostBuf {
+    void* p = nullptr;
+    size_t bytes = 0;
+    cudaEvent_t done = nullptr;
+    cudaError_t ensure(size_t want);
+    void release();
+    HostBuf() = default;
+    HostBuf(const HostBuf&) = delete;
+    HostBuf& operator=(const HostBuf&) = delete;
+    ~HostBuf() { release(); }
+};
+
 struct BvhMeta;
 
 // What a traversal kernel needs; the root index is read on the device from the
@@ -196,6 +210,7 @@ struct gr_ctx {
     // of gr_trace_host's pipeline); error word at offset 64
     gr::DevBuf counter;
     gr::DevBuf stage_in, stage_out;  // device staging for the host-memory entry points
+    gr::HostBuf image[2];            // page-locked chunks of gr_render's host image (3 MB each at most)
     // 8-wide layout build state, reused by every BVH of the context (grown,
     // never shrunk, until the context is destroyed); the render server's
     // thread may build too, so it is taken under its lock

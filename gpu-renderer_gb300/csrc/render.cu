@@ -38,9 +38,9 @@ constexpr float kShadowTmin = 0.0f, kShadowTmax = 0.9999f;
 inline uint32_t draws_before(int b) { return b == 0 ? 2u : 9u * (uint32_t)b + 1u; }
 constexpr int kShadeThreads = 256;
 constexpr int kShadowBase = kMaxDepth + 1;  // shadow queue counters start here
-constexpr int kErrWord = 2 * kMaxDepth + 4;
-constexpr int kBinBase = 2 * kMaxDepth + 8;  // kShadeBins counters per bounce start here
-constexpr int kCntWords = kBinBase + kShadeBins * (kMaxDepth + 1);
+constexpr int kBinBase = 2 * kMaxDepth + 4;  // kShadeBins counters per bounce start here
+constexpr int kCntWords = (kBinBase + kShadeBins * (kMaxDepth + 1) + 1) & ~1;  // even: the work counters follow
+constexpr size_t kCounterBytes = sizeof(uint32_t) * kCntWords + sizeof(unsigned long long) * (kMaxDepth + 1);
 
 __device__ __forceinline__ uint32_t lane_lt() {
     uint32_t m;
@@ -390,7 +390,7 @@ __global__ void __launch_bounds__(trav::kMaxTraceThreads, 4) k_trace_wave(Paths 
     WaveSrc<LAYOUT> src{(b & 1) ? ps.ray[1] : ps.ray[0], ps.sray, ps.scon, ps.hit, ps.acc, ps.jobs, nc,
                         (uint64_t)nc + ns, ps.hdr->njobs == 1, b == 0 ? kCameraTmin : kScatterTmin,
                         b == 0 ? kCameraTmax : kScatterTmax};
-    trav::traverse_loop<trav::kMixed, LAYOUT, SSTACK, trav::kRefillQueue>(src, ps.work + b, ps.cnt + kErrWord, s_stack);
+    trav::traverse_loop<trav::kMixed, LAYOUT, SSTACK, trav::kRefillQueue>(src, ps.work + b, &ps.hdr->err, s_stack);
 }
 
 // ---- shading groups -----------------------------------------------------------------
@@ -612,6 +612,22 @@ __global__ void __launch_bounds__(kShadeThreads) k_resolve(Paths ps) {
     for (uint32_t j = threadIdx.x; j < h.njobs; j += blockDim.x) s_base[j] = ps.jobs[j].pix_base;
     if (threadIdx.x == 0) s_base[h.njobs] = h.total_pix;
     __syncthreads();
+    if (blockIdx.x == gridDim.x - 1 && threadIdx.x < 32) {  // the wave's ray counts, added to the running totals
+        unsigned long long c = 0, sh = 0;
+        for (uint32_t b = threadIdx.x; b <= h.max_depth; b += 32) {
+            c += ps.cnt[b];
+            if (b < h.max_depth) sh += ps.cnt[kShadowBase + b];
+        }
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1) {
+            c += __shfl_xor_sync(0xFFFFFFFFu, c, d);
+            sh += __shfl_xor_sync(0xFFFFFFFFu, sh, d);
+        }
+        if (threadIdx.x == 0) {
+            ps.hdr->closest_rays = h.closest_rays + c;
+            ps.hdr->shadow_rays = h.shadow_rays + sh;
+        }
+    }
     const uint32_t stride = gridDim.x * blockDim.x;
     for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < h.total_pix; r += stride) {
         const JobDev& J = ps.jobs[find_job(s_base, h.njobs, r)];
@@ -653,42 +669,27 @@ __global__ void __launch_bounds__(kShadeThreads) k_filter(const double* __restri
     }
 }
 
-// Mean linear radiance per pixel (3 floats), the same arithmetic as the host
-// read-back of gr_render: sum * (1 / count) in double, rounded to float.
+// Mean linear radiance per pixel (3 floats): sum * (1 / count) in double,
+// rounded to float. One value a thread, so that stores to host memory, which
+// cross the host link, go out as whole 128-byte lines.
 __global__ void __launch_bounds__(kShadeThreads) k_mean_rgb(const double* __restrict__ fb,
                                                             const uint32_t* __restrict__ fbc, uint32_t npix,
                                                             float* __restrict__ out) {
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < npix; i += gridDim.x * blockDim.x) {
-        const uint32_t n = fbc[i];
-        const double inv = n ? 1.0 / (double)n : 0.0;
-#pragma unroll
-        for (int c = 0; c < 3; ++c) out[3ull * i + c] = (float)(fb[3ull * i + c] * inv);
+    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < 3ull * npix; i += stride) {
+        const uint32_t n = fbc[i / 3];
+        out[i] = (float)(fb[i] * (n ? 1.0 / (double)n : 0.0));
     }
 }
 
-__global__ void k_wave_end(Paths ps) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    WaveHeader* h = ps.hdr;
-    unsigned long long c = 0, sh = 0;
-    for (uint32_t b = 0; b <= h->max_depth; ++b) c += ps.cnt[b];
-    for (uint32_t b = 0; b < h->max_depth; ++b) sh += ps.cnt[kShadowBase + b];
-    h->closest_rays += c;
-    h->shadow_rays += sh;
-}
-
 // One wave: clear counters, camera rays, depth_steps x (trace, shade)
-// (steps past the wave's max_depth return at once), resolve, ray counts.
+// (steps past the wave's max_depth return at once), resolve (which adds the ray counts up).
 template <int LAYOUT, int SSTACK>
 cudaError_t issue_wave_l(const Paths& ps, uint32_t depth_steps, int tgrid, int tblock, int sgrid, bool bin,
                          cudaStream_t s) {
     const size_t smem = trav::traverse_smem(LAYOUT, SSTACK, tblock);
     cudaError_t e;
-    const size_t cnt_bytes = sizeof(uint32_t) * (2 * kMaxDepth + 4);
-    const size_t bin_bytes = sizeof(uint32_t) * (kCntWords - kBinBase);
-    const size_t work_bytes = sizeof(unsigned long long) * (2 * kMaxDepth + 4);
-    if ((e = cudaMemsetAsync(ps.cnt, 0, cnt_bytes, s)) != cudaSuccess) return e;
-    if (bin && (e = cudaMemsetAsync(ps.cnt + kBinBase, 0, bin_bytes, s)) != cudaSuccess) return e;
-    if ((e = cudaMemsetAsync(ps.work, 0, work_bytes, s)) != cudaSuccess) return e;
+    if ((e = cudaMemsetAsync(ps.cnt, 0, kCounterBytes, s)) != cudaSuccess) return e;
     k_camera<<<sgrid, kShadeThreads, 0, s>>>(ps);
     for (int b = 0; b <= (int)depth_steps; ++b) {
         k_trace_wave<LAYOUT, SSTACK><<<tgrid, tblock, smem, s>>>(ps, b);
@@ -701,7 +702,6 @@ cudaError_t issue_wave_l(const Paths& ps, uint32_t depth_steps, int tgrid, int t
         }
     }
     k_resolve<<<sgrid, kShadeThreads, 0, s>>>(ps);
-    k_wave_end<<<1, 32, 0, s>>>(ps);
     return cudaGetLastError();
 }
 
@@ -747,6 +747,9 @@ uint64_t mix64(uint64_t h, uint64_t v) {
 
 size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 
+// a wave's header fields and job table as the host stages them
+constexpr size_t kWaveBytes = (sizeof(WaveHeader) + sizeof(JobDev) * kMaxJobs + 255) & ~size_t(255);
+
 size_t path_layout(uint32_t cap, char* base, Paths* ps) {
     size_t off = 0;
     auto take = [&](size_t bytes) {
@@ -762,10 +765,10 @@ size_t path_layout(uint32_t cap, char* base, Paths* ps) {
     ps->bins = (uint32_t*)take(4 * ((kShadeBins + 1) / 2) * c);
     ps->sray = (float4*)take(32 * c);
     ps->scon = (float4*)take(16 * c);
-    ps->cnt = (uint32_t*)take(sizeof(uint32_t) * kCntWords);
-    ps->work = (unsigned long long*)take(sizeof(unsigned long long) * (2 * kMaxDepth + 4));
-    ps->hdr = (WaveHeader*)take(sizeof(WaveHeader));
-    ps->jobs = (JobDev*)take(sizeof(JobDev) * kMaxJobs);
+    ps->cnt = (uint32_t*)take(kCounterBytes);  // counters and work counters, cleared as one
+    ps->work = (unsigned long long*)(ps->cnt + kCntWords);
+    ps->hdr = (WaveHeader*)take(sizeof(WaveHeader) + sizeof(JobDev) * kMaxJobs);
+    ps->jobs = (JobDev*)(ps->hdr + 1);
     ps->capacity = cap;
     return off;
 }
@@ -792,19 +795,19 @@ void WavePool::release() {
             cudaEventDestroy(ev[i]);
             ev[i] = nullptr;
         }
-    if (h_jobs) cudaFreeHost(h_jobs);
-    if (h_hdr) cudaFreeHost(h_hdr);
-    h_jobs = nullptr;
-    h_hdr = nullptr;
+    if (h_wave) cudaFreeHost(h_wave);
+    if (h_result) cudaFreeHost(h_result);
+    h_wave = nullptr;
+    h_result = nullptr;
     mem.release();
     capacity = 0;
 }
 
 cudaError_t WavePool::ensure(uint32_t paths) {
     cudaError_t e;
-    if (!h_jobs) {
-        if ((e = cudaMallocHost((void**)&h_jobs, sizeof(JobDev) * kMaxJobs * kSlots)) != cudaSuccess) return e;
-        if ((e = cudaMallocHost((void**)&h_hdr, sizeof(WaveHeader) * kSlots)) != cudaSuccess) return e;
+    if (!h_wave) {
+        if (!h_result && (e = cudaMallocHost((void**)&h_result, sizeof(WaveHeader))) != cudaSuccess) return e;
+        if ((e = cudaMallocHost((void**)&h_wave, kWaveBytes * kSlots)) != cudaSuccess) return e;
         for (int i = 0; i < kSlots; ++i)
             if ((e = cudaEventCreateWithFlags(&ev[i], cudaEventDisableTiming)) != cudaSuccess) return e;
     }
@@ -819,15 +822,16 @@ cudaError_t WavePool::ensure(uint32_t paths) {
     }
     path_layout(paths, (char*)mem.p, &ps);
     capacity = paths;
-    if ((e = cudaMemset(ps.hdr, 0, sizeof(WaveHeader))) != cudaSuccess) return e;
-    return cudaMemset(ps.cnt + kErrWord, 0, 4);
+    return cudaMemset(ps.hdr, 0, sizeof(WaveHeader));
 }
 
-cudaError_t WavePool::clear_errors(cudaStream_t s) {
-    return mem.p ? cudaMemsetAsync(ps.cnt + kErrWord, 0, 4, s) : cudaSuccess;
+cudaError_t WavePool::begin_call(cudaStream_t s) {
+    return cudaMemsetAsync(ps.hdr, 0, offsetof(WaveHeader, njobs), s);
 }
 
-const uint32_t* WavePool::error_word() const { return ps.cnt + kErrWord; }
+cudaError_t WavePool::end_call(cudaStream_t s) {
+    return cudaMemcpyAsync(h_result, ps.hdr, sizeof(WaveHeader), cudaMemcpyDeviceToHost, s);
+}
 
 uint32_t pack_wave(std::vector<HostJob*>& jobs, uint32_t capacity, std::vector<JobDev>& out, uint32_t* total_paths,
                    uint32_t* total_pix, uint32_t* max_depth) {
@@ -873,7 +877,7 @@ cudaError_t filter_rgba8(const double* fb, const uint32_t* fbc, uint32_t npix, u
 
 cudaError_t mean_rgb(const double* fb, const uint32_t* fbc, uint32_t npix, float* out, cudaStream_t s) {
     if (npix == 0) return cudaSuccess;
-    const int grid = (int)std::min<uint32_t>((npix + kShadeThreads - 1) / kShadeThreads, 4096u);
+    const int grid = (int)std::min<uint64_t>((3ull * npix + kShadeThreads - 1) / kShadeThreads, 4096u);
     k_mean_rgb<<<grid, kShadeThreads, 0, s>>>(fb, fbc, npix, out);
     return cudaGetLastError();
 }
@@ -895,18 +899,17 @@ cudaError_t run_wave(WavePool& pool, const JobDev* h_jobs, uint32_t njobs, uint3
     const int slot = pool.slot;
     pool.slot = (pool.slot + 1) % WavePool::kSlots;
     if ((e = cudaEventSynchronize(pool.ev[slot])) != cudaSuccess) return e;
-    JobDev* stage = pool.h_jobs + (size_t)slot * kMaxJobs;
-    std::memcpy(stage, h_jobs, sizeof(JobDev) * njobs);
-    WaveHeader& h = pool.h_hdr[slot];
-    h = WaveHeader{};
+    WaveHeader h{};
     h.njobs = njobs;
     h.total_paths = total_paths;
     h.total_pix = total_pix;
     h.max_depth = max_depth;
-    if ((e = cudaMemcpyAsync(ps.jobs, stage, sizeof(JobDev) * njobs, cudaMemcpyHostToDevice, s)) != cudaSuccess)
-        return e;
-    // the header's running ray totals stay on the device; only the wave fields are written
-    if ((e = cudaMemcpyAsync(ps.hdr, &h, offsetof(WaveHeader, closest_rays), cudaMemcpyHostToDevice, s)) != cudaSuccess)
+    char* stage = pool.h_wave + (size_t)slot * kWaveBytes;
+    constexpr size_t at = offsetof(WaveHeader, njobs);  // the running totals before it stay on the device
+    std::memcpy(stage, (const char*)&h + at, sizeof(h) - at);
+    std::memcpy(stage + sizeof(h) - at, h_jobs, sizeof(JobDev) * njobs);
+    if ((e = cudaMemcpyAsync((char*)ps.hdr + at, stage, sizeof(h) - at + sizeof(JobDev) * njobs,
+                             cudaMemcpyHostToDevice, s)) != cudaSuccess)
         return e;
     if ((e = cudaEventRecord(pool.ev[slot], s)) != cudaSuccess) return e;
     const int tgrid = num_sms * occ;

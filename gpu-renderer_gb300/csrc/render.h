@@ -87,15 +87,20 @@ struct JobDev {
     uint64_t seed;
 };
 
-// Device-resident description of the current wave (written by the host
-// before each wave; the captured kernel sequence reads it).
+// Device-resident state of a pool's waves. The first part accumulates on the
+// device (and is read back, or cleared, as one copy); the second describes the
+// current wave and is written by the host before each wave, together with the
+// job table right behind it, as one copy; the captured kernel sequence reads it.
 struct WaveHeader {
-    uint32_t njobs;
+    unsigned long long closest_rays, shadow_rays;  // running totals
+    uint32_t err;        // device error bits (ERR_*)
+    uint32_t pad[3];
+    uint32_t njobs;      // from here on written per wave
     uint32_t total_paths;
     uint32_t total_pix;
     uint32_t max_depth;  // bounces the wave runs (max over its jobs)
-    unsigned long long closest_rays, shadow_rays;  // running totals
 };
+static_assert(sizeof(WaveHeader) == 48 && alignof(JobDev) <= 16, "the job table follows the header");
 
 // Path state for one wave. What the next bounce needs of a path (its ray and
 // throughput) lives at the path's place in the bounce's queue, not at its path
@@ -153,17 +158,17 @@ struct WavePool {
     static constexpr int kGraphs = 4;
     WaveGraph graphs[kGraphs];
     void release_graphs();
-    // pinned staging for the per-wave job table and header, one slot per wave
+    // pinned staging for the per-wave header and job table, one slot per wave
     // in flight; a slot is rewritten only after its event has completed
-    JobDev* h_jobs = nullptr;
-    WaveHeader* h_hdr = nullptr;
+    char* h_wave = nullptr;
+    WaveHeader* h_result = nullptr;  // pinned: what a call reads back
     cudaEvent_t ev[kSlots] = {};
     int slot = 0;
     cudaError_t ensure(uint32_t paths);
-    // clears the device error bits before a call, on stream s
-    cudaError_t clear_errors(cudaStream_t s);
-    // device address of the error bits (ERR_*), read back after a call
-    const uint32_t* error_word() const;
+    // A call's waves: begin clears the ray totals and error bits, end starts the
+    // read-back of both into h_result (valid once the stream has been waited for).
+    cudaError_t begin_call(cudaStream_t s);
+    cudaError_t end_call(cudaStream_t s);
     void release();
     ~WavePool() { release(); }
 };
@@ -219,7 +224,8 @@ uint32_t pack_wave(std::vector<HostJob*>& jobs, uint32_t capacity, std::vector<J
 // Mean radiance -> sRGB-encoded RGBA8 (R in the low byte), the reference's
 // filter_kernel (pathtracer_kernel.h:792-810); pixels without samples are black.
 cudaError_t filter_rgba8(const double* fb, const uint32_t* fbc, uint32_t npix, uint32_t* out, cudaStream_t s);
-// Mean radiance of an accumulation into 3 floats per pixel in device memory.
+// Mean radiance of an accumulation into 3 floats per pixel in memory the device
+// can write (device memory, or page-locked host memory).
 cudaError_t mean_rgb(const double* fb, const uint32_t* fbc, uint32_t npix, float* out, cudaStream_t s);
 
 }  // namespace gr

@@ -123,9 +123,7 @@ extern "C" gr_status gr_render_batch(gr_ctx* ctx, gr_scene* const* scenes, const
         return cuda_status(e);
     }
     cudaStream_t s = ctx->stream;
-    if ((e = pool.clear_errors(s)) != cudaSuccess) return cuda_status(e);
-    gr::WaveHeader before{};
-    cudaMemcpyAsync(&before, pool.ps.hdr, sizeof(before), cudaMemcpyDeviceToHost, s);
+    if ((e = pool.begin_call(s)) != cudaSuccess) return cuda_status(e);
     std::vector<gr::JobDev> table;
     uint32_t waves = 0;
     const bool graph = !(n && (opts[0].flags & GR_RENDER_NO_GRAPH));
@@ -142,11 +140,10 @@ extern "C" gr_status gr_render_batch(gr_ctx* ctx, gr_scene* const* scenes, const
         }
         ++waves;
     }
-    gr::WaveHeader after{};
-    uint32_t err = 0;
-    cudaMemcpyAsync(&after, pool.ps.hdr, sizeof(after), cudaMemcpyDeviceToHost, s);
-    cudaMemcpyAsync(&err, pool.error_word(), 4, cudaMemcpyDeviceToHost, s);
+    if ((e = pool.end_call(s)) != cudaSuccess) return cuda_status(e);
     if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return cuda_status(e);
+    const gr::WaveHeader& after = *pool.h_result;
+    const uint32_t err = after.err;
     uint64_t samples = 0;
     for (uint32_t i = 0; i < n; ++i) {
         scenes[i]->samples_done += opts[i].spp;
@@ -154,8 +151,8 @@ extern "C" gr_status gr_render_batch(gr_ctx* ctx, gr_scene* const* scenes, const
     }
     if (stats) {
         stats->ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
-        stats->closest_rays = after.closest_rays - before.closest_rays;
-        stats->shadow_rays = after.shadow_rays - before.shadow_rays;
+        stats->closest_rays = after.closest_rays;
+        stats->shadow_rays = after.shadow_rays;
         stats->samples = samples;
         stats->waves = waves;
         stats->device_errors = err;
