@@ -17,11 +17,12 @@
 // summed, and the children become the next level at consecutive indices, so
 // a node's inner children are contiguous from child_base and its leaf
 // triangles contiguous from tri_base (copied into the layout's own triangle
-// array). The numbering is deterministic; the host reads one level size per
-// level.
+// array). The numbering is deterministic. All levels run in one cooperative
+// launch; the host reads the sizes once, at its end.
 #include <algorithm>
 
 #include "gr_internal.h"
+#include "grid_sync.cuh"
 #include "quant.cuh"
 
 namespace gr {
@@ -29,16 +30,12 @@ namespace {
 
 using namespace q8;
 
-constexpr int kBlock8 = 256;
-constexpr int kLanesPerNode = 8;            // lanes collapsing one 8-wide node
-constexpr int kNodesPerCollapseBlock = 32;  // nodes per collapse block: one emit warp
-constexpr int kCollapseThreads = kNodesPerCollapseBlock * kLanesPerNode;
-constexpr int kScanThreads = 1024;
+constexpr int kThreads8 = 256;
+constexpr int kWarps8 = kThreads8 / 32;
+constexpr int kLanesPerNode = 8;                  // lanes collapsing one 8-wide node
+constexpr int kNodesPerWarp = 32 / kLanesPerNode;
 constexpr int32_t kEmptySlot = INT32_MIN;
-constexpr int kMaxLevels8 = 72;
-constexpr int kLevelsPerSync = 4;        // levels launched per host read-back of the level state
-constexpr int kCollapseBlocksPerSm = 5;  // grid of the collapse (its loop covers any level size)
-constexpr int kEmitBlocksPerSm = 4;
+constexpr uint32_t kMaxLevels8 = 72;
 
 // 8-wide planes: plane(q) = q * 2^e + lo, taken EXACTLY (the traversal
 // measures it as fma(q, 2^e / d, (lo - o) / d) with error margins, never
@@ -66,8 +63,9 @@ __device__ __forceinline__ int pick_exponent8(float lo, float hi, uint32_t* err)
     const float extent = __fsub_rn(hi, lo);
     int e = -126;
     if (extent > 0.0f) {
-        int ex;
-        frexpf(__fdiv_rn(extent, 255.0f), &ex);
+        const float q = __fdiv_rn(extent, 255.0f);
+        int ex = (int)(__float_as_uint(q) >> 23) - 126;  // q = m * 2^ex with m in [1/2, 1)
+        if (ex <= -126 || ex >= 129) frexpf(q, &ex);     // subnormal or infinite
         e = max(-126, min(kMaxExp8, ex - 1));
     }
     while (cmp_plane(255, pow2f(e), lo, hi) < 0) {
@@ -80,18 +78,42 @@ __device__ __forceinline__ int pick_exponent8(float lo, float hi, uint32_t* err)
     return e;
 }
 
-__device__ __forceinline__ uint32_t quant_lo8(float v, float scale, float lo) {
-    int q = 0;
-    for (int step = 128; step > 0; step >>= 1)  // largest q with plane(q) <= v (plane(0) = lo <= v)
-        if (q + step <= 255 && cmp_plane(q + step, scale, lo, v) <= 0) q += step;
+__device__ __forceinline__ bool finite(float x) { return fabsf(x) <= 3.402823466e38f; }
+
+// Largest q with plane(q) <= v and smallest q with plane(q) >= v, by search (any input).
+__device__ __noinline__ uint32_t quant_search8(float v, float scale, float lo, bool upper) {
+    int q = upper ? 255 : 0;
+    for (int step = 128; step > 0; step >>= 1) {
+        if (!upper && q + step <= 255 && cmp_plane(q + step, scale, lo, v) <= 0) q += step;
+        if (upper && q - step >= 0 && cmp_plane(q - step, scale, lo, v) >= 0) q -= step;
+    }
     return (uint32_t)q;
 }
 
-__device__ __forceinline__ uint32_t quant_hi8(float v, float scale, float lo) {
-    int q = 255;
-    for (int step = 128; step > 0; step >>= 1)  // smallest q with plane(q) >= v (plane(255) >= v)
-        if (q - step >= 0 && cmp_plane(q - step, scale, lo, v) >= 0) q -= step;
-    return (uint32_t)q;
+// The same for lo <= v <= plane(255) (v may be NaN, as the search takes it) and
+// lo, plane(255) finite: x = (v - lo) / scale is rounded once, by the
+// subtraction (inv = 1 / scale is a power of two), and rounding keeps order, so
+// its floor or ceiling can be off only when x is a whole number, and then the
+// sign of the subtraction's error (two-sum) decides. A nonzero difference whose
+// quotient underflows to 0 lies above plane(0).
+__device__ __forceinline__ uint32_t quant_lo8(float v, float inv, float lo) {
+    const float d = __fsub_rn(v, lo), x = __fmul_rn(d, inv);
+    const float f = __fadd_rd(x, 8388608.0f);  // 2^23 + floor(x)
+    const float b = __fsub_rn(d, v);           // two-sum of v and -lo
+    const float err = __fsub_rn(__fsub_rn(v, __fsub_rn(d, b)), __fadd_rn(lo, b));
+    const bool exact = __fsub_rn(f, 8388608.0f) == x;
+    const uint32_t q = __float_as_uint(f) & 0xFFu;
+    return exact && err < 0.0f ? q - 1u : (isnan(x) ? 0u : q);
+}
+
+__device__ __forceinline__ uint32_t quant_hi8(float v, float inv, float lo) {
+    const float d = __fsub_rn(v, lo), x = __fmul_rn(d, inv);
+    const float f = __fadd_ru(x, 8388608.0f);  // 2^23 + ceil(x)
+    const float b = __fsub_rn(d, v);
+    const float err = __fsub_rn(__fsub_rn(v, __fsub_rn(d, b)), __fadd_rn(lo, b));
+    const bool exact = __fsub_rn(f, 8388608.0f) == x;
+    const uint32_t q = __float_as_uint(f) & 0xFFu;
+    return exact && (err > 0.0f || (q == 0u && d > 0.0f)) ? q + 1u : (isnan(x) ? 0u : q);
 }
 
 __device__ __forceinline__ float half_area(const CBox& b) {
@@ -101,31 +123,35 @@ __device__ __forceinline__ float half_area(const CBox& b) {
     return __fadd_rn(__fadd_rn(__fmul_rn(dx, dy), __fmul_rn(dy, dz)), __fmul_rn(dz, dx));
 }
 
-// One level of the build as the device sees it: its node count, where its
-// nodes start in the output, where its leaf triangles start, and whether a
-// capacity was exceeded (the build then stops with no more writes). Level l's
-// scan writes level l + 1's state, so the host launches levels without reading
-// their sizes back.
-struct Level8 {
-    uint32_t n, out_base, tri_cursor, overflow;
+// What the host reads back: nodes and leaf triangles written, and whether a
+// capacity was exceeded (the build then stopped with no more writes).
+struct Size8 {
+    uint32_t nodes, tris, overflow, pad;
 };
 
-__global__ void k8_init(const BvhMeta* __restrict__ meta, uint32_t* frontier, Level8* level,
-                        unsigned long long* bsum) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        frontier[0] = meta->root;
-        level[0] = Level8{1u, 0u, 0u, 0u};
-        bsum[0] = 0ull;
-    }
-}
+struct Build8 {
+    const Node* nodes;
+    const Tri* tris;
+    const BvhMeta* meta;
+    uint32_t* frontier[2];     // binary ids of a level's nodes, levels alternate
+    int32_t* slots;            // 8 child references per node of the level, by slot
+    unsigned long long* bsum;  // per block: inner children | leaves << 32 of its nodes
+    Node8Q* out;               // nodes [0, cap) go here (the layout's own array, kept from an earlier build)
+    uint32_t cap;
+    Node8Q* rest;              // nodes [cap, ..) here (scratch, same indices)
+    Tri* tris8;
+    uint32_t max_nodes, max_tris, num_tris;
+    Size8* size;
+    uint32_t* sync;
+    uint32_t* err;
+};
 
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
-// Order-preserving 32-bit key of a float (larger float, larger key); -0 and +0
-// share one key, as they compare equal.
-__device__ __forceinline__ uint32_t order_key(float x) {
-    const uint32_t b = __float_as_uint(x == 0.0f ? 0.0f : x);
-    return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
+__device__ __forceinline__ uint32_t group_max(uint32_t x) {
+#pragma unroll
+    for (int d = 1; d < kLanesPerNode; d <<= 1) x = max(x, __shfl_xor_sync(0xFFFFFFFFu, x, d));
+    return x;
 }
 
 // Eight lanes per 8-wide node, four nodes per warp: lane k of a group holds
@@ -133,120 +159,135 @@ __device__ __forceinline__ uint32_t order_key(float x) {
 // candidates in order would make it (first largest on ties), so the node does
 // not depend on the lanes' arithmetic order. Loops run the same number of
 // times in every group, so each shuffle has the whole warp. Writes the node
-// (without its bases) and its 8 slot references when `have`; returns the
-// counts (inner | leaf << 32).
-__device__ unsigned long long collapse_group(const Node* __restrict__ nodes, bool have, uint32_t root_id,
-                                             Node8Q* __restrict__ out, int32_t* __restrict__ sref_out, uint32_t* err) {
+// (without its bases) through the warp's shared records `rec` and its 8 slot
+// references when `have`; adds the warp's inner children and leaves to the counts.
+__device__ __forceinline__ void collapse_group(const Build8& B, bool have, uint32_t root_id, Node8Q* __restrict__ out,
+                                               int32_t* __restrict__ sref_out, uint32_t (*rec)[24], int32_t (*sref)[8],
+                                               uint32_t& inner, uint32_t& leaves) {
     constexpr uint32_t kAll = 0xFFFFFFFFu;
     constexpr int W = kLanesPerNode;
-    const int k = threadIdx.x & (W - 1);
+    const int lane = threadIdx.x & 31, k = lane & (W - 1), g = lane / W;
     int32_t ref = kEmptySlot;
     CBox box = {{0.0f, 0.0f, 0.0f}, {0.0f, 0.0f, 0.0f}};
+    float lo[3] = {0.0f, 0.0f, 0.0f}, hi[3] = {0.0f, 0.0f, 0.0f};
     int cnt8 = 0;
     if (have) {
-        const Node root = nodes[root_id];
+        const Node root = B.nodes[root_id];
         box = child_box(root, k & 1);
         if (k < 2) ref = k ? root.q3.y : root.q3.x;
         cnt8 = 2;
+        // the node's box: its binary children's boxes are the exact minima and
+        // maxima of everything below, whatever is opened
+        const CBox b0 = child_box(root, 0), b1 = child_box(root, 1);
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            lo[a] = fminf(b0.lo[a], b1.lo[a]);
+            hi[a] = fmaxf(b0.hi[a], b1.hi[a]);
+        }
     }
     // an inner candidate's node is fetched towards L2 as soon as it becomes a
     // candidate, so opening it later waits on L2 rather than DRAM
-    if (ref >= 0) prefetch_l2(nodes + ref);
-    // open the inner candidate with the largest surface area (at most 6 times)
+    if (ref >= 0) prefetch_l2(B.nodes + ref);
+    // open the inner candidate with the largest surface area (at most 6 times);
+    // scanned in order a NaN area is kept only when it comes first
     for (int step = 0; step < 6; ++step) {
+        const bool cand = ref >= 0;  // lanes past cnt8 hold no reference
+        const uint32_t cands = (__ballot_sync(kAll, cand) >> (g * W)) & 0xFFu;
+        const bool open = cands != 0 && cnt8 < 8;
+        if (!__any_sync(kAll, open)) break;
+        // areas are +0 .. inf or NaN, whose bits are in order as integers
         const float area = half_area(box);
-        int best = -1;
-        float best_a = 0.0f;
-        for (int j = 0; j < W; ++j) {
-            const float aj = __shfl_sync(kAll, area, j, W);
-            const int32_t rj = __shfl_sync(kAll, ref, j, W);
-            if (j < cnt8 && rj >= 0 && (best < 0 || aj > best_a)) {
-                best = j;
-                best_a = aj;
-            }
+        uint32_t key = cand ? __float_as_uint(area) : 0u;
+        if (isnan(area)) key = cand && k == __ffs(cands) - 1 ? 0xFFFFFFFFu : 0u;
+        const uint32_t top = group_max(key);
+        const uint32_t at = (__ballot_sync(kAll, cand && key == top) >> (g * W)) & 0xFFu;
+        const int best = __ffs(at) - 1;
+        const int32_t rb = __shfl_sync(kAll, ref, max(best, 0), W);
+        if (open && (k == best || k == cnt8)) {
+            // the opened lane takes the first child, the next free one the second
+            const float4* nd = reinterpret_cast<const float4*>(B.nodes + rb);
+            const int c = k == best ? 0 : 1;
+            const float4 xy = __ldg(nd + c);
+            const float2 z = __ldg(reinterpret_cast<const float2*>(nd + 2) + c);
+            ref = __ldg(reinterpret_cast<const int32_t*>(nd + 3) + c);
+            box.lo[0] = xy.x; box.hi[0] = xy.y; box.lo[1] = xy.z; box.hi[1] = xy.w; box.lo[2] = z.x; box.hi[2] = z.y;
+            if (ref >= 0) prefetch_l2(B.nodes + ref);
         }
-        const int32_t rb = __shfl_sync(kAll, ref, best < 0 ? 0 : best, W);
-        if (best >= 0 && cnt8 < 8) {
-            const Node cn = nodes[rb];
-            if (k == best) {
-                ref = cn.q3.x;
-                box = child_box(cn, 0);
-            }
-            if (k == cnt8) {
-                ref = cn.q3.y;
-                box = child_box(cn, 1);
-            }
-            if ((k == best || k == cnt8) && ref >= 0) prefetch_l2(nodes + ref);
-            ++cnt8;
-        }
+        if (open) ++cnt8;
     }
-    // node box (folded in candidate order) and centre (lo + hi)
-    float lo[3], hi[3], nc[3];
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        lo[a] = __shfl_sync(kAll, box.lo[a], 0, W);
-        hi[a] = __shfl_sync(kAll, box.hi[a], 0, W);
-    }
-#pragma unroll
-    for (int j = 1; j < W; ++j) {
-#pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            const float l = __shfl_sync(kAll, box.lo[a], j, W), h = __shfl_sync(kAll, box.hi[a], j, W);
-            if (j < cnt8) {
-                lo[a] = fminf(lo[a], l);
-                hi[a] = fmaxf(hi[a], h);
-            }
-        }
-    }
-#pragma unroll
-    for (int a = 0; a < 3; ++a) nc[a] = __fadd_rn(lo[a], hi[a]);
     // this lane's child scored against every slot
-    const float dx = __fsub_rn(__fadd_rn(box.lo[0], box.hi[0]), nc[0]);
-    const float dy = __fsub_rn(__fadd_rn(box.lo[1], box.hi[1]), nc[1]);
-    const float dz = __fsub_rn(__fadd_rn(box.lo[2], box.hi[2]), nc[2]);
+    const float dx = __fsub_rn(__fadd_rn(box.lo[0], box.hi[0]), __fadd_rn(lo[0], hi[0]));
+    const float dy = __fsub_rn(__fadd_rn(box.lo[1], box.hi[1]), __fadd_rn(lo[1], hi[1]));
+    const float dz = __fsub_rn(__fadd_rn(box.lo[2], box.hi[2]), __fadd_rn(lo[2], hi[2]));
     float sc[8];
-    bool nan_score = false;
+    bool odd_score = false;  // infinite or NaN
 #pragma unroll
     for (int s = 0; s < 8; ++s) {
         sc[s] = __fadd_rn(__fadd_rn((s & 1) ? dx : -dx, (s & 2) ? dy : -dy), (s & 4) ? dz : -dz);
-        nan_score |= isnan(sc[s]);
+        odd_score |= !finite(sc[s]);
     }
-    const bool slow = __any_sync(kAll, k < cnt8 && nan_score);
-    // greedy assignment: the best (score, then lowest child, then lowest slot) first
+    // greedy assignment: the best (score, then lowest child, then lowest slot)
+    // first. That order is strict, so a pair that is the best left of its child
+    // and the best left of its slot is one the greedy rule takes: a round takes
+    // all such pairs of the node at once (two or three rounds instead of eight).
+    // Lane s also holds column s of the scores (an 8 x 8 transpose). Taken rows
+    // and columns score -inf, below every finite score.
     uint32_t used = 0;
-    bool taken = false;
     int my_slot = -1;
-    for (int it = 0; it < 8; ++it) {
-        int win = -1;
-        if (!slow) {
-            // this lane's first largest free slot, then the group's largest
-            // score with the lowest pair 8 k + s on ties (-0 and +0 tie)
-            const bool cand = k < cnt8 && !taken;
-            int bs = -1;
-            float bsc = 0.0f;
+    if (!__any_sync(kAll, k < cnt8 && odd_score)) {
+        if (k >= cnt8) {
 #pragma unroll
-            for (int s = 0; s < 8; ++s)
-                if (cand && !(used >> s & 1u) && (bs < 0 || sc[s] > bsc)) {
-                    bs = s;
-                    bsc = sc[s];
-                }
-            uint32_t key = bs >= 0 ? order_key(bsc) : 0u;
-            int p = bs >= 0 ? 8 * k + bs : 0xFF;
+            for (int s = 0; s < 8; ++s) sc[s] = -INFINITY;
+        }
+        float col[8];
 #pragma unroll
-            for (int d = 1; d < W; d <<= 1) {
-                const uint32_t ok = __shfl_xor_sync(kAll, key, d, W);
-                const int op = __shfl_xor_sync(kAll, p, d, W);
-                if (ok > key || (ok == key && op < p)) {
-                    key = ok;
-                    p = op;
-                }
+        for (int s = 0; s < 8; ++s) col[s] = sc[s];
+#pragma unroll
+        for (int d = 1; d < W; d <<= 1) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                if (i & d) continue;
+                const float got = __shfl_xor_sync(kAll, (k & d) ? col[i] : col[i ^ d], d);
+                if (k & d) col[i] = got;
+                else col[i ^ d] = got;
             }
-            win = p;
-        } else {
-            // a NaN score in the warp: fold the group's pairs in order, as one thread would
+        }
+        uint32_t left = (1u << cnt8) - 1u;  // children without a slot
+        for (int round = 0; round < 8; ++round) {  // each round takes at least the best pair left of every node
+            if (!__any_sync(kAll, left != 0)) break;
+            const float rm = fmaxf(fmaxf(fmaxf(sc[0], sc[1]), fmaxf(sc[2], sc[3])),
+                                   fmaxf(fmaxf(sc[4], sc[5]), fmaxf(sc[6], sc[7])));
+            const float cm = fmaxf(fmaxf(fmaxf(col[0], col[1]), fmaxf(col[2], col[3])),
+                                   fmaxf(fmaxf(col[4], col[5]), fmaxf(col[6], col[7])));
+            int rs = 7, cs = 7;  // the first slot of this child's best, the first child of this slot's
+#pragma unroll
+            for (int s = 6; s >= 0; --s) {
+                rs = sc[s] == rm ? s : rs;
+                cs = col[s] == cm ? s : cs;
+            }
+            const int mate = __shfl_sync(kAll, cs, rs, W);  // the best child of this child's best slot
+            const int back = __shfl_sync(kAll, rs, cs, W);  // the best slot of this slot's best child
+            const bool row = (left >> k & 1u) && mate == k;
+            const bool column = !(used >> k & 1u) && (left >> cs & 1u) && back == k;
+            const uint32_t rows = (__ballot_sync(kAll, row) >> (g * W)) & 0xFFu;
+            const uint32_t columns = (__ballot_sync(kAll, column) >> (g * W)) & 0xFFu;
+            if (row) my_slot = rs;
+            left &= ~rows;
+            used |= columns;
+#pragma unroll
+            for (int s = 0; s < 8; ++s) {
+                if (columns >> s & 1u) sc[s] = -INFINITY;
+                if (rows >> s & 1u) col[s] = -INFINITY;
+            }
+        }
+        if (left != 0 && k == 0) atomicOr(B.err, ERR_RANGE);  // cannot happen
+    } else {
+        // an infinite or NaN score in the warp: fold the group's pairs in order, as one thread would
+        for (int it = 0; it < 8; ++it) {
+            int win = -1;
             float wsc = 0.0f;
             for (int j = 0; j < W; ++j) {
-                const bool tj = __shfl_sync(kAll, (int)taken, j, W) != 0;
+                const bool tj = __shfl_sync(kAll, my_slot, j, W) >= 0;
 #pragma unroll
                 for (int s = 0; s < 8; ++s) {
                     const float x = __shfl_sync(kAll, sc[s], j, W);
@@ -256,199 +297,173 @@ __device__ unsigned long long collapse_group(const Node* __restrict__ nodes, boo
                     }
                 }
             }
-        }
-        if (it < cnt8) {
-            if (win < 0 || win >= 64) {  // no free pair: cannot happen while it < cnt8 <= 8
-                if (k == 0) atomicOr(err, ERR_RANGE);
-            } else {
+            if (it < cnt8 && win >= 0) {
                 used |= 1u << (win & 7);
-                if (k == (win >> 3)) {
-                    taken = true;
-                    my_slot = win & 7;
-                }
+                if (k == (win >> 3)) my_slot = win & 7;
             }
         }
     }
     // quantise: per-axis exponents (lanes 0-2), then this lane's child's six planes
     uint32_t my_be = 0;
     if (have && k < 3) my_be = (uint32_t)(pick_exponent8(k == 0 ? lo[0] : (k == 1 ? lo[1] : lo[2]),
-                                                         k == 0 ? hi[0] : (k == 1 ? hi[1] : hi[2]), err) + 127);
+                                                         k == 0 ? hi[0] : (k == 1 ? hi[1] : hi[2]), B.err) + 127);
     uint32_t be[3];
-    float scale[3];
 #pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        be[a] = __shfl_sync(kAll, my_be, a, W);
-        scale[a] = __uint_as_float(be[a] << 23);
-    }
-    uint32_t wq[12];
+    for (int a = 0; a < 3; ++a) be[a] = __shfl_sync(kAll, my_be, a, W);
+    const bool child = k < cnt8 && my_slot >= 0;
+    uint32_t imask = child && ref >= 0 ? 1u << my_slot : 0u;
 #pragma unroll
-    for (int w = 0; w < 12; ++w) wq[w] = 0;
-    if (k < cnt8 && my_slot >= 0) {
-        const int sh = 8 * (my_slot & 3), half = my_slot >> 2;
+    for (int d = 1; d < W; d <<= 1) imask |= __shfl_xor_sync(kAll, imask, d, W);
+    // the node's 24 words through shared memory: each child drops its bytes
+    uint32_t* r = rec[g];
+    int32_t* sr = sref[g];
+    __syncwarp();  // the records of the warp's last nodes have been read
+#pragma unroll
+    for (int j = 0; j < 3; ++j) r[k + 8 * j] = 0u;
+    sr[k] = kEmptySlot;
+    __syncwarp();
+    if (child) {
+        unsigned char* q = reinterpret_cast<unsigned char*>(r + 8);
+        bool plain = true;  // finite planes that reach the node's corner
+#pragma unroll
+        for (int a = 0; a < 3; ++a) plain &= finite(lo[a]) && finite(hi[a]) && be[a] < (uint32_t)(kMaxExp8 + 127);
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
-            const uint32_t ql = quant_lo8(box.lo[a], scale[a], lo[a]) << sh;
-            const uint32_t qh = quant_hi8(box.hi[a], scale[a], lo[a]) << sh;
-            wq[4 * a + 0] = half ? 0u : ql;
-            wq[4 * a + 1] = half ? ql : 0u;
-            wq[4 * a + 2] = half ? 0u : qh;
-            wq[4 * a + 3] = half ? qh : 0u;
+            const float scale = __uint_as_float(be[a] << 23), inv = __uint_as_float((254u - be[a]) << 23);
+            q[16 * a + my_slot] = (unsigned char)(plain ? quant_lo8(box.lo[a], inv, lo[a])
+                                                        : quant_search8(box.lo[a], scale, lo[a], false));
+            q[16 * a + 8 + my_slot] = (unsigned char)(plain ? quant_hi8(box.hi[a], inv, lo[a])
+                                                            : quant_search8(box.hi[a], scale, lo[a], true));
         }
+        sr[my_slot] = ref;
     }
-    uint32_t imask = (k < cnt8 && ref >= 0 && my_slot >= 0) ? 1u << my_slot : 0u;
+    if (k < 3) r[k] = __float_as_uint(k == 0 ? lo[0] : (k == 1 ? lo[1] : lo[2]));
+    if (k == 3) r[3] = be[0] | (be[1] << 8) | (be[2] << 16) | (imask << 24);
+    if (k == 6) r[6] = used;
+    __syncwarp();
+    if (have) {
+        uint32_t* o = reinterpret_cast<uint32_t*>(out);
 #pragma unroll
-    for (int d = 1; d < W; d <<= 1) {
-        imask |= __shfl_xor_sync(kAll, imask, d, W);
-#pragma unroll
-        for (int w = 0; w < 12; ++w) wq[w] |= __shfl_xor_sync(kAll, wq[w], d, W);
+        for (int j = 0; j < 3; ++j) o[k + 8 * j] = r[k + 8 * j];
+        sref_out[k] = sr[k];
     }
-    if (!have) return 0ull;
-    // the node's 24 words: lane k writes words k, k + 8 and k + 16
-    uint32_t w0 = 0, w1 = 0, w2 = 0;
-    if (k < 3) w0 = __float_as_uint(k == 0 ? lo[0] : (k == 1 ? lo[1] : lo[2]));
-    if (k == 3) w0 = be[0] | (be[1] << 8) | (be[2] << 16) | (imask << 24);
-    if (k == 6) w0 = used;
-#pragma unroll
-    for (int w = 0; w < 8; ++w) {
-        if (k == w) w1 = wq[w];
-        if (k == w && w < 4) w2 = wq[8 + w];
-    }
-    uint32_t* o = reinterpret_cast<uint32_t*>(out);
-    o[k] = w0;
-    o[k + 8] = w1;
-    o[k + 16] = w2;
-    // slot references: each child at its slot, empty slots marked
-    if (k < cnt8 && my_slot >= 0) sref_out[my_slot] = ref;
-    if (!(used >> k & 1u)) sref_out[k] = kEmptySlot;
-    const uint32_t n_inner = __popc(imask);
-    return (unsigned long long)n_inner | ((unsigned long long)(cnt8 - n_inner) << 32);
+    inner += __popc(__ballot_sync(kAll, child && ref >= 0));
+    leaves += __popc(__ballot_sync(kAll, child && ref < 0));
 }
 
-// The level's nodes, eight lanes each (four per warp), over a grid of any
-// size; each node's counts go to cnt[i] and are added into the sum of its
-// 32-node tile (bsum, zeroed by the previous level's scan).
-__global__ void __launch_bounds__(kCollapseThreads) k8_collapse(const Node* __restrict__ nodes,
-                                                              const uint32_t* __restrict__ frontier,
-                                                              const Level8* __restrict__ level,
-                                                              Node8Q* __restrict__ out, int32_t* __restrict__ slots,
-                                                              unsigned long long* __restrict__ cnt,
-                                                              unsigned long long* __restrict__ bsum, uint32_t* err) {
-    const Level8 L = *level;
-    constexpr uint32_t kPerWarp = 32 / kLanesPerNode;
-    const uint32_t warps = gridDim.x * (kCollapseThreads / 32);
-    const uint32_t g = (threadIdx.x & 31) / kLanesPerNode;
-    for (uint32_t w = blockIdx.x * (kCollapseThreads / 32) + threadIdx.x / 32; (uint64_t)w * kPerWarp < L.n;
-         w += warps) {  // the same trip count for the whole warp
-        const uint32_t i = w * kPerWarp + g;
-        const bool have = i < L.n;
-        const unsigned long long c =
-            collapse_group(nodes, have, have ? frontier[i] : 0u, out + L.out_base + i, slots + 8ull * i, err);
-        if (have && (threadIdx.x & (kLanesPerNode - 1)) == 0) {
-            cnt[i] = c;
-            atomicAdd(&bsum[i / kNodesPerCollapseBlock], c);
-        }
-    }
-}
-
-// Exclusive scan of the level's tile sums in place (one block); writes the
-// next level's state and zeroes the next level's tile sums.
-__global__ void __launch_bounds__(kScanThreads) k8_scan_blocks(unsigned long long* bsum, const Level8* level,
-                                                               Level8* next, unsigned long long* next_bsum,
-                                                               uint32_t max_nodes, uint32_t max_tris) {
-    __shared__ unsigned long long s_warp[32];
-    __shared__ uint32_t s_next_tiles;
-    const Level8 L = *level;
-    const uint32_t nblocks = (L.n + kNodesPerCollapseBlock - 1) / kNodesPerCollapseBlock;
-    const uint32_t per = (nblocks + kScanThreads - 1) / kScanThreads;
-    const uint32_t b0 = threadIdx.x * per, b1 = min(nblocks, b0 + per);
-    unsigned long long sum = 0;
-    for (uint32_t b = b0; b < b1; ++b) sum += bsum[b];
-    // exclusive scan of the threads' sums: within each warp, then over the warp totals
-    static_assert(kScanThreads == 1024, "32 warps of 32");
+// The whole build. Per level: each warp collapses a run of consecutive nodes
+// (four at a time) and counts their children; a grid barrier; every block sums
+// the blocks before it, and each warp gives its nodes' children their places
+// (a ballot over a step's 32 slots ranks them: inner children become the next
+// level, leaf triangles are copied); a second barrier. Small levels go to as
+// few warps a block as they need, on all blocks, so their few nodes run on many
+// SMs. One launch replaces three a level and a host read-back every four: the
+// 1M-triangle soup (8 levels, 284 Ki nodes) takes 0.21 ms instead of 0.49, and a
+// rebuilt BVH with 262,144 rays against it 877 us instead of 1,131. A small level
+// costs 11 us (collapsing one node 5 us of dependent loads, two barriers 4.5, the
+// places 1.8); the 242 Ki-node level 60 to 90 us a block, issue bound (1,240 warp
+// instructions for four nodes; 1,510 before the slots were assigned in rounds and
+// the planes quantised without a search). 4 blocks an SM (59 registers) against
+// 3: 877 and 886 us; prefetching the next nodes' neighbourhoods to L1 or L2
+// changed nothing.
+__global__ void __launch_bounds__(kThreads8, 4) k8_build(Build8 B) {
+    __shared__ uint32_t s_rec[kWarps8][kNodesPerWarp][24];
+    __shared__ int32_t s_ref[kWarps8][kNodesPerWarp][8];
+    __shared__ unsigned long long s_warp[kWarps8], s_before[kWarps8], s_total[kWarps8];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    unsigned long long x = sum;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-        const unsigned long long y = __shfl_up_sync(0xFFFFFFFFu, x, d);
-        if (lane >= d) x += y;
-    }
-    if (lane == 31) s_warp[warp] = x;
-    __syncthreads();
-    if (warp == 0) {
-        unsigned long long w = s_warp[lane];
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const unsigned long long y = __shfl_up_sync(0xFFFFFFFFu, w, d);
-            if (lane >= d) w += y;
-        }
-        s_warp[lane] = w;
-    }
-    __syncthreads();
-    unsigned long long run = (warp ? s_warp[warp - 1] : 0ull) + x - sum;
-    for (uint32_t b = b0; b < b1; ++b) {
-        const unsigned long long v = bsum[b];
-        bsum[b] = run;
-        run += v;
-    }
-    if (threadIdx.x == 0) {
-        const unsigned long long total = s_warp[31];
-        Level8 nx;
-        nx.n = (uint32_t)total;
-        nx.out_base = L.out_base + L.n;
-        nx.tri_cursor = L.tri_cursor + (uint32_t)(total >> 32);
-        nx.overflow = L.overflow;
-        if ((uint64_t)nx.out_base + nx.n > max_nodes || nx.tri_cursor > max_tris) {
-            nx.overflow = 1u;
-            nx.n = 0u;
-        }
-        *next = nx;
-        s_next_tiles = (nx.n + kNodesPerCollapseBlock - 1) / kNodesPerCollapseBlock;
-    }
-    __syncthreads();
-    for (uint32_t b = threadIdx.x; b < s_next_tiles; b += kScanThreads) next_bsum[b] = 0ull;
-}
-
-// Writes each node's bases, the next level's binary ids (inner children in
-// slot order) and the leaf triangles (in slot order) into the layout's
-// triangle array. A node's offsets are its tile's exclusive count sum plus the
-// counts of the nodes before it in the tile, whose 32 nodes are one warp here
-// (a warp scan). Nothing is written once a capacity was exceeded.
-__global__ void __launch_bounds__(kBlock8) k8_emit(const Level8* __restrict__ level, const Level8* __restrict__ next,
-                                                   Node8Q* __restrict__ out, const int32_t* __restrict__ slots,
-                                                   const unsigned long long* __restrict__ cnt,
-                                                   const unsigned long long* __restrict__ bsum,
-                                                   uint32_t* __restrict__ next_frontier, const Tri* __restrict__ tris,
-                                                   Tri* __restrict__ tris8) {
-    static_assert(kNodesPerCollapseBlock == 32, "a tile's nodes are one emit warp");
-    const Level8 L = *level;
-    if (next->overflow) return;
-    const uint32_t next_base = L.out_base + L.n;
-    const int lane = threadIdx.x & 31;
-    for (uint32_t base = blockIdx.x * kBlock8; base < L.n; base += gridDim.x * kBlock8) {  // block-uniform
-        const uint32_t i = base + threadIdx.x;
-        const unsigned long long c = i < L.n ? cnt[i] : 0ull;
-        unsigned long long x = c;
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const unsigned long long y = __shfl_up_sync(0xFFFFFFFFu, x, d);
-            if (lane >= d) x += y;
-        }
-        if (i >= L.n) continue;
-        const unsigned long long pre = bsum[i / kNodesPerCollapseBlock] + (x - c);
-        const uint32_t inner0 = (uint32_t)pre, leaf0 = (uint32_t)(pre >> 32);
-        out[L.out_base + i].child_base = next_base + inner0;
-        out[L.out_base + i].tri_base = L.tri_cursor + leaf0;
-        uint32_t ri = 0, rl = 0;
-        for (int s = 0; s < 8; ++s) {
-            const int32_t r = slots[8ull * i + s];
-            if (r == kEmptySlot) continue;
-            if (r >= 0) {
-                next_frontier[inner0 + ri++] = (uint32_t)r;
-            } else {
-                tris8[L.tri_cursor + leaf0 + rl++] = tris[(uint32_t)(~r)];
+    const uint32_t g = lane / kLanesPerNode, k = lane & (kLanesPerNode - 1);
+    const uint32_t grid = gridDim.x;
+    uint32_t n = 1, out_base = 0, tri_cursor = 0, arrived = 0, overflow = 0;
+    for (uint32_t level = 0; n != 0; ++level) {
+        const uint32_t* frontier = (level & 1) ? B.frontier[1] : B.frontier[0];
+        const uint64_t per_block = (uint64_t)grid * kNodesPerWarp;
+        const uint32_t active = (uint32_t)min((uint64_t)kWarps8, (n + per_block - 1) / per_block);  // warps a block
+        const uint64_t steps = ((uint64_t)n + per_block * active - 1) / (per_block * active);
+        const uint64_t first = ((uint64_t)blockIdx.x * active + warp) * steps * kNodesPerWarp;
+        const uint32_t begin = (uint32_t)warp < active ? (uint32_t)min((uint64_t)n, first) : n;
+        const uint32_t end = (uint32_t)warp < active ? (uint32_t)min((uint64_t)n, first + steps * kNodesPerWarp) : n;
+        uint32_t inner = 0, leaves = 0;
+        for (uint32_t base = begin; base < end; base += kNodesPerWarp) {  // the same trip count for the whole warp
+            const uint32_t i = base + g;
+            bool have = i < end;
+            const uint32_t id = !have ? 0u : (level == 0 ? B.meta->root : __ldcg(frontier + i));
+            if (have && id >= B.max_nodes) {
+                atomicOr(B.err, ERR_RANGE);
+                have = false;
             }
+            const uint32_t at = out_base + i;
+            collapse_group(B, have, id, (at < B.cap ? B.out : B.rest) + at, B.slots + 8ull * i, s_rec[warp],
+                           s_ref[warp], inner, leaves);
         }
+        if (lane == 0) s_warp[warp] = (unsigned long long)inner | ((unsigned long long)leaves << 32);
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            unsigned long long sum = 0;
+            for (int w = 0; w < kWarps8; ++w) sum += s_warp[w];
+            B.bsum[blockIdx.x] = sum;
+        }
+        grid_barrier(B.sync, ++arrived * grid, B.err);
+        unsigned long long before = 0, total = 0;
+        for (uint32_t j = threadIdx.x; j < grid; j += kThreads8) {
+            const unsigned long long v = __ldcg(B.bsum + j);
+            total += v;
+            if (j < blockIdx.x) before += v;
+        }
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1) {
+            before += __shfl_xor_sync(0xFFFFFFFFu, before, d);
+            total += __shfl_xor_sync(0xFFFFFFFFu, total, d);
+        }
+        if (lane == 0) {
+            s_before[warp] = before;
+            s_total[warp] = total;
+        }
+        __syncthreads();
+        before = 0;
+        total = 0;
+        for (int w = 0; w < kWarps8; ++w) {
+            before += s_before[w];
+            total += s_total[w];
+            if (w < warp) before += s_warp[w];
+        }
+        const uint32_t next_base = out_base + n;
+        const uint64_t next_n = (uint32_t)total, next_tri = tri_cursor + (total >> 32);
+        if (next_base + next_n > B.max_nodes || next_tri > B.max_tris || level >= kMaxLevels8) {
+            overflow = 1;  // the same for every block
+            break;
+        }
+        uint32_t in_run = (uint32_t)before, leaf_run = (uint32_t)(before >> 32);
+        uint32_t* next = (level & 1) ? B.frontier[0] : B.frontier[1];
+        for (uint32_t base = begin; base < end; base += kNodesPerWarp) {
+            const uint32_t i = base + g;
+            const bool have = i < end;
+            const int32_t r = have ? B.slots[8ull * i + k] : kEmptySlot;
+            const uint32_t mi = __ballot_sync(0xFFFFFFFFu, r >= 0);
+            const uint32_t ml = __ballot_sync(0xFFFFFFFFu, r < 0 && r != kEmptySlot);
+            const uint32_t lt = (1u << lane) - 1u, gt = (1u << (g * kLanesPerNode)) - 1u;  // lanes before, groups before
+            if (have && k == 0) {
+                const uint32_t at = out_base + i;
+                Node8Q* nd = (at < B.cap ? B.out : B.rest) + at;
+                *reinterpret_cast<uint2*>(&nd->child_base) =
+                    make_uint2(next_base + in_run + __popc(mi & gt), tri_cursor + leaf_run + __popc(ml & gt));
+            }
+            if (r >= 0) {
+                const uint32_t to = in_run + __popc(mi & lt);
+                if (to < B.max_nodes) next[to] = (uint32_t)r;
+            } else if (r != kEmptySlot) {
+                const uint32_t to = tri_cursor + leaf_run + __popc(ml & lt), from = (uint32_t)(~r);
+                if (to < B.max_tris && from < B.num_tris) B.tris8[to] = B.tris[from];
+                else atomicOr(B.err, ERR_RANGE);
+            }
+            in_run += __popc(mi);
+            leaf_run += __popc(ml);
+        }
+        grid_barrier(B.sync, ++arrived * grid, B.err);
+        out_base = next_base;
+        tri_cursor = (uint32_t)next_tri;
+        n = (uint32_t)next_n;
     }
+    if (blockIdx.x == 0 && threadIdx.x == 0) *B.size = Size8{out_base, tri_cursor, overflow, 0u};
 }
 
 size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
@@ -461,64 +476,78 @@ cudaError_t bvh8_build(BvhBuffers& b, uint32_t n, DevBuf& scratch, int num_sms, 
     if (n == 0) return cudaSuccess;
     const size_t maxnodes = n > 1 ? n - 1 : 1;
     const size_t maxtris = std::max<size_t>(n, 2);  // a lone triangle fills both children of its node
-    const size_t maxtiles = (maxnodes + kNodesPerCollapseBlock - 1) / kNodesPerCollapseBlock;
-    // scratch: two frontiers, slot refs, counts, two sets of tile sums, the
-    // level states, and the nodes before compaction
+    // resident blocks: the launch's barriers need every block on the GPU at once
+    int dev = 0, coop = 0, per_sm = 0;
+    cudaError_t e;
+    if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
+    if ((e = cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev)) != cudaSuccess) return e;
+    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k8_build, kThreads8, 0)) != cudaSuccess) return e;
+    // a level has at most n - 1 nodes, four to a warp and step
+    uint32_t grid = (uint32_t)std::min<size_t>(std::max(1, num_sms) * (size_t)std::max(1, per_sm),
+                                               (maxnodes + kNodesPerWarp - 1) / kNodesPerWarp);
+    if (!coop) grid = 1;
+    // scratch: two frontiers, slot refs, block sums, sizes and barrier counter, the nodes
     size_t off = 0;
     const size_t o_f0 = off; off += align256(4 * maxnodes);
     const size_t o_f1 = off; off += align256(4 * maxnodes);
     const size_t o_sl = off; off += align256(32 * maxnodes);
-    const size_t o_cn = off; off += align256(8 * maxnodes);
-    const size_t o_b0 = off; off += align256(8 * maxtiles);
-    const size_t o_b1 = off; off += align256(8 * maxtiles);
-    const size_t o_lv = off; off += align256(sizeof(Level8) * (kMaxLevels8 + 1));
+    const size_t o_bs = off; off += align256(8 * (size_t)grid);
+    const size_t o_sz = off; off += 256;  // Size8, then the barrier counter at 64
     const size_t o_nd = off; off += align256(sizeof(Node8Q) * maxnodes);
-    cudaError_t e;
     if ((e = scratch.ensure(off)) != cudaSuccess) return e;
     if ((e = b.tris8.ensure(sizeof(Tri) * maxtris)) != cudaSuccess) return e;
     char* base = (char*)scratch.p;
-    uint32_t* frontier[2] = {(uint32_t*)(base + o_f0), (uint32_t*)(base + o_f1)};
-    int32_t* slots = (int32_t*)(base + o_sl);
-    unsigned long long* cnt = (unsigned long long*)(base + o_cn);
-    unsigned long long* tile_sums[2] = {(unsigned long long*)(base + o_b0), (unsigned long long*)(base + o_b1)};
-    Level8* level_state = (Level8*)(base + o_lv);
-    Node8Q* staged = (Node8Q*)(base + o_nd);
-    const Node* nodes = (const Node*)b.nodes.p;
-    uint32_t* err = &((BvhMeta*)b.meta.p)->err;
-    const int sms = std::max(1, num_sms);
-    k8_init<<<1, 32, 0, s>>>((const BvhMeta*)b.meta.p, frontier[0], level_state, tile_sums[0]);
-    // levels are launched kLevelsPerSync at a time; the host reads the state
-    // after each batch and stops at the first empty level (launches past it do
-    // nothing)
-    Level8 h{};
-    int level = 0;
+    Build8 B;
+    B.nodes = (const Node*)b.nodes.p;
+    B.tris = (const Tri*)b.tris.p;
+    B.meta = (const BvhMeta*)b.meta.p;
+    B.frontier[0] = (uint32_t*)(base + o_f0);
+    B.frontier[1] = (uint32_t*)(base + o_f1);
+    B.slots = (int32_t*)(base + o_sl);
+    B.bsum = (unsigned long long*)(base + o_bs);
+    B.out = (Node8Q*)b.nodes8.p;
+    B.cap = b.nodes8.p ? (uint32_t)std::min<size_t>(b.nodes8.bytes / sizeof(Node8Q), maxnodes) : 0u;
+    B.rest = (Node8Q*)(base + o_nd);
+    B.tris8 = (Tri*)b.tris8.p;
+    B.max_nodes = (uint32_t)maxnodes;
+    B.max_tris = (uint32_t)maxtris;
+    B.num_tris = n;
+    B.size = (Size8*)(base + o_sz);
+    B.sync = (uint32_t*)(base + o_sz + 64);
+    B.err = &((BvhMeta*)b.meta.p)->err;
+    if ((e = cudaMemsetAsync(base + o_sz, 0, 256, s)) != cudaSuccess) return e;
     for (;;) {
-        for (int j = 0; j < kLevelsPerSync && level < kMaxLevels8; ++j, ++level) {
-            const int c = level & 1;
-            k8_collapse<<<sms * kCollapseBlocksPerSm, kCollapseThreads, 0, s>>>(
-                nodes, frontier[c], level_state + level, staged, slots, cnt, tile_sums[c], err);
-            k8_scan_blocks<<<1, kScanThreads, 0, s>>>(tile_sums[c], level_state + level, level_state + level + 1,
-                                                      tile_sums[c ^ 1], (uint32_t)maxnodes, (uint32_t)maxtris);
-            k8_emit<<<sms * kEmitBlocksPerSm, kBlock8, 0, s>>>(level_state + level, level_state + level + 1, staged,
-                                                              slots, cnt, tile_sums[c], frontier[c ^ 1],
-                                                              (const Tri*)b.tris.p, (Tri*)b.tris8.p);
+        if (grid == 1) {  // a lone block meets nobody at its barriers
+            k8_build<<<1, kThreads8, 0, s>>>(B);
+            e = cudaGetLastError();
+        } else {
+            void* args[] = {&B};
+            e = cudaLaunchCooperativeKernel((const void*)k8_build, dim3(grid), dim3(kThreads8), args, 0, s);
         }
-        if ((e = cudaGetLastError()) != cudaSuccess) return e;
-        if ((e = cudaMemcpyAsync(&h, level_state + level, sizeof(h), cudaMemcpyDeviceToHost, s)) != cudaSuccess)
+        if (e != cudaErrorCooperativeLaunchTooLarge) break;
+        (void)cudaGetLastError();  // e.g. a client held to part of the SMs
+        grid = (grid + 1) / 2;
+    }
+    if (e != cudaSuccess) return e;
+    Size8 h{};
+    if ((e = cudaMemcpyAsync(&h, B.size, sizeof(h), cudaMemcpyDeviceToHost, s)) != cudaSuccess) return e;
+    if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return e;
+    if (h.overflow) return cudaErrorInvalidValue;
+    if (h.nodes > B.cap) {  // the layout's array grows: what it held stays in place
+        DevBuf grown;
+        if ((e = grown.ensure(sizeof(Node8Q) * h.nodes)) != cudaSuccess) return e;
+        if (B.cap && (e = cudaMemcpyAsync(grown.p, b.nodes8.p, sizeof(Node8Q) * B.cap, cudaMemcpyDeviceToDevice, s)) !=
+                         cudaSuccess)
+            return e;
+        if ((e = cudaMemcpyAsync((Node8Q*)grown.p + B.cap, B.rest + B.cap, sizeof(Node8Q) * (h.nodes - B.cap),
+                                 cudaMemcpyDeviceToDevice, s)) != cudaSuccess)
             return e;
         if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return e;
-        if (h.overflow) return cudaErrorInvalidValue;
-        if (h.n == 0) break;
-        if (level >= kMaxLevels8) return cudaErrorInvalidValue;
+        std::swap(grown.p, b.nodes8.p);
+        std::swap(grown.bytes, b.nodes8.bytes);
     }
-    const uint32_t out_base = h.out_base, tri_cursor = h.tri_cursor;
-    if ((e = b.nodes8.ensure(sizeof(Node8Q) * out_base)) != cudaSuccess) return e;
-    if ((e = cudaMemcpyAsync(b.nodes8.p, staged, sizeof(Node8Q) * out_base, cudaMemcpyDeviceToDevice, s)) !=
-        cudaSuccess)
-        return e;
-    if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return e;
-    b.count8 = out_base;
-    b.tris8_count = tri_cursor;
+    b.count8 = h.nodes;
+    b.tris8_count = h.tris;
     return cudaSuccess;
 }
 

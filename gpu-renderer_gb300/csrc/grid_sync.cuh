@@ -1,0 +1,38 @@
+// Bounded device-side waits shared by the builders (lbvh.cu, bvh8.cu).
+#pragma once
+
+#include "gr_internal.h"
+
+namespace gr {
+
+__device__ __forceinline__ uint32_t ld_acquire(const uint32_t* p) {
+    uint32_t v;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+
+// Grid-wide barrier of a cooperative launch (every block resident): block
+// arrivals are counted on `ctr`, and the k-th barrier of the launch waits for
+// (k + 1) * gridDim.x arrivals, at most `limit` polls (then ERR_TIMEOUT).
+// The block barrier before the fence puts every thread's writes ahead of the
+// arrival; the block barrier after it puts the other blocks' writes ahead of
+// every thread's later reads (which go to L2: __ldcg).
+__device__ __forceinline__ void grid_barrier(uint32_t* ctr, uint32_t target, uint32_t* err,
+                                             uint32_t limit = kSpinLimit) {
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        atomicAdd(ctr, 1u);
+        uint32_t spins = 0;
+        while (ld_acquire(ctr) < target) {
+            if (++spins > limit) {
+                atomicOr(err, ERR_TIMEOUT);
+                break;
+            }
+        }
+        __threadfence();
+    }
+    __syncthreads();
+}
+
+}  // namespace gr

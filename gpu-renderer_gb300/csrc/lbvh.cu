@@ -13,6 +13,7 @@
 #include <cuda.h>  // CUcontext / CUresult: the driver entry points are reached through the runtime
 
 #include "gr_internal.h"
+#include "grid_sync.cuh"
 
 namespace gr {
 namespace {
@@ -23,11 +24,6 @@ constexpr int kRefitChunk = 256;
 
 // ---- small device helpers ---------------------------------------------------
 
-__device__ __forceinline__ uint32_t ld_acquire(const uint32_t* p) {
-    uint32_t v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
 __device__ __forceinline__ void st_release(uint32_t* p, uint32_t v) {
     asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
@@ -260,30 +256,6 @@ __device__ __forceinline__ uint32_t match_digit(uint32_t d) {
 constexpr uint32_t kSumTiles = 64;
 
 constexpr size_t kOsSmem = sizeof(uint32_t) * (kOsWarps * 256 + 256 + 256 + 2 * kOsTile + 2 * kOsWarps + 1);
-
-// Grid-wide barrier of a cooperative launch (every block resident): block
-// arrivals are counted on `ctr`, and the k-th barrier of the launch waits for
-// (k + 1) * gridDim.x arrivals, at most `limit` polls (then ERR_TIMEOUT).
-// The block barrier before the fence puts every thread's writes ahead of the
-// arrival; the block barrier after it puts the other blocks' writes ahead of
-// every thread's later reads (which go to L2: __ldcg).
-__device__ __forceinline__ void grid_barrier(uint32_t* ctr, uint32_t target, uint32_t* err,
-                                             uint32_t limit = kSpinLimit) {
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();
-        atomicAdd(ctr, 1u);
-        uint32_t spins = 0;
-        while (ld_acquire(ctr) < target) {
-            if (++spins > limit) {
-                atomicOr(err, ERR_TIMEOUT);
-                break;
-            }
-        }
-        __threadfence();
-    }
-    __syncthreads();
-}
 
 // One tile of one sort pass: ranks the tile's keys by the pass's digit, finds
 // where each digit's run of the tile starts in the output, and writes the

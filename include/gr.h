@@ -154,7 +154,7 @@ gr_status gr_bvh_export(gr_bvh* bvh, uint32_t* h_sorted_prim, uint32_t* h_sorted
  *                      leaf triangles copied into node order
  * The binary tree is always built; another layout is derived from it on the
  * GPU when first requested and kept until the next build (the 8-wide build
- * waits for the stream once per tree level). */
+ * waits for the stream). */
 #define GR_LAYOUT_BVH2 0
 #define GR_LAYOUT_BVH4 1
 #define GR_LAYOUT_BVH4_Q8 2
