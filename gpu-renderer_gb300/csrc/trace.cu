@@ -47,12 +47,12 @@ struct RaySrc {
 template <bool ANY, int LAYOUT, int SSTACK>
 __global__ void __launch_bounds__(trav::kMaxTraceThreads, 4) k_trace(const void* __restrict__ nodes, const Tri* __restrict__ tris,
                                                                   const BvhMeta* __restrict__ meta,
-                                                                  const float4* __restrict__ rays, uint64_t n,
+                                                                  const float4* __restrict__ rays, uint64_t n, uint32_t lanes,
                                                                   float4* __restrict__ hits, unsigned long long* counter,
                                                                   uint32_t* err) {
     extern __shared__ int2 s_stack[];
     RaySrc src{rays, hits, n, nodes, tris, meta->root};
-    trav::traverse_loop<ANY ? trav::kAny : trav::kClosest, LAYOUT, SSTACK, trav::kRefillRays>(src, counter, err, s_stack);
+    trav::traverse_loop<ANY ? trav::kAny : trav::kClosest, LAYOUT, SSTACK, trav::kRefillRays>(src, lanes, counter, err, s_stack);
 }
 
 template <bool ANY, int LAYOUT, int SSTACK>
@@ -67,10 +67,12 @@ cudaError_t launch(const BvhDevice& bvh, const void* nodes, int block, const flo
         if (e != cudaSuccess) return e;
         if (occ[bi] < 1) occ[bi] = 1;
     }
-    const uint64_t warps_needed = (n + 31) / 32;
+    const uint32_t warps = (uint32_t)(num_sms * occ[bi] * (block / 32));
+    const uint32_t lanes = trav::lanes_per_warp(n, warps);
+    const uint64_t warps_needed = (n + lanes - 1) / lanes;
     const uint64_t blocks_needed = (warps_needed + block / 32 - 1) / (block / 32);
     const int grid = (int)std::min<uint64_t>((uint64_t)num_sms * occ[bi], blocks_needed);
-    k_trace<ANY, LAYOUT, SSTACK><<<grid, block, smem, s>>>(nodes, bvh.tris, bvh.meta, r, n, h, counter, err);
+    k_trace<ANY, LAYOUT, SSTACK><<<grid, block, smem, s>>>(nodes, bvh.tris, bvh.meta, r, n, lanes, h, counter, err);
     return cudaGetLastError();
 }
 

@@ -583,6 +583,22 @@ __device__ __forceinline__ bool trace_step(L_& L, int2* s_stack, int2* l_stack, 
 constexpr int kRefillRays = 4;
 constexpr int kRefillQueue = 12;
 
+// Lanes of a warp that take rays, for n rays on at most `warps` resident warps: a
+// launch that cannot give every lane of half the GPU's warps a ray spreads its
+// rays over more warps. A short launch lasts as long as its longest ray, and a
+// ray's step lasts as long as what the other lanes of its warp do in it (leaf
+// tests above all); more warps than half the resident ones made the issue slots
+// the limit instead. Incoherent rays in 100 k triangles, 32 lanes against this rule
+// against one ray for every resident warp first (us): binary nodes 1,021 rays
+// 192 / 119 / 119, 10,000 230 / 167 / 175, 50,000 242 / 226 / 247; 8-wide nodes
+// 1,021 rays 103 / 66 / 67, 10,000 126 / 105 / 112, 50,000 135 / 140 / 174. A
+// 160 x 120 x 1 spp preview 615 -> 460 us.
+constexpr uint32_t kSpread = 2;
+__host__ __device__ inline uint32_t lanes_per_warp(uint64_t n, uint32_t warps) {
+    const uint64_t per = (kSpread * n + warps - 1) / warps;
+    return per >= 32 ? 32u : (per < 1 ? 1u : (uint32_t)per);
+}
+
 // Persistent dynamic-fetch loop. `Src` supplies the work:
 //   Index                                             integer type of a ray's index
 //   n                                                 number of rays
@@ -599,7 +615,8 @@ constexpr int kRefillQueue = 12;
 // (traverse_smem). Every thread of the block calls it (the table is filled
 // behind a block barrier).
 template <int Q, int LAYOUT, int SSTACK, int REFILL, class Src>
-__device__ __forceinline__ void traverse_loop(Src& src, unsigned long long* counter, uint32_t* err, int2* s_stack) {
+__device__ __forceinline__ void traverse_loop(Src& src, uint32_t lanes, unsigned long long* counter, uint32_t* err,
+                                              int2* s_stack) {
     int2 l_stack[kStackMax - SSTACK];
     // 8-wide layout: xor_permute8 as a table (octant x mask, 2 KB after the
     // short stacks), filled once per block
@@ -612,6 +629,9 @@ __device__ __forceinline__ void traverse_loop(Src& src, unsigned long long* coun
     const uint32_t ltmask = lanemask_lt();
     using Index = typename Src::Index;
     const uint64_t n = src.n;
+    // lanes past `lanes` stay idle; they count towards the threshold
+    const int surplus = 32 - (int)lanes;
+    const int refill = surplus + min(REFILL, (int)lanes);
     Lane<Index> L;
     bool active = false;
     bool exhausted = false;
@@ -620,12 +640,13 @@ __device__ __forceinline__ void traverse_loop(Src& src, unsigned long long* coun
         const int nidle = __popc(idle);
         if (exhausted) {
             if (nidle == 32) break;  // a refill that found no rays leaves every lane idle
-        } else if (nidle >= REFILL || nidle == 32) {
+        } else if (nidle >= refill) {
             unsigned long long base = 0;
-            if (lane == 0) base = atomicAdd(counter, (unsigned long long)nidle);
+            const int want = nidle - surplus;
+            if (lane == 0) base = atomicAdd(counter, (unsigned long long)want);
             base = __shfl_sync(0xFFFFFFFFu, base, 0);
-            if (base + nidle >= n) exhausted = true;
-            if (!active) {
+            if (base + want >= n) exhausted = true;
+            if (!active && lane < (int)lanes) {
                 const uint64_t i = base + __popc(idle & ltmask);
                 if (i < n) {
                     float4 r0, r1;
