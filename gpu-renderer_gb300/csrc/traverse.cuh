@@ -381,6 +381,21 @@ __device__ __forceinline__ float2 plane_pair(uint32_t w0, uint32_t w1, int b, fl
     return t;
 }
 
+// (a0 - b0, a1 - b1) in one packed subtraction, each rounded as a scalar one.
+__device__ __forceinline__ float2 sub2(float a0, float a1, float b0, float b1) {
+    float2 r;
+    asm("{\n\t"
+        ".reg .b64 a, b, r;\n\t"
+        "mov.b64 a, {%2, %3};\n\t"
+        "mov.b64 b, {%4, %5};\n\t"
+        "sub.rn.f32x2 r, a, b;\n\t"
+        "mov.b64 {%0, %1}, r;\n\t"
+        "}"
+        : "=f"(r.x), "=f"(r.y)
+        : "f"(a0), "f"(a1), "f"(b0), "f"(b1));
+    return r;
+}
+
 // Per node and axis, with S = 2^e * (1/d) and C = (lo - o) * (1/d): the
 // plane scale S' = 2^15 * S (exact) and the near / far offsets C' -+ m with
 // C' = C - S' and m = |C| * 2^-20 + |S| * 2^-7. The roundings of C, C', the
@@ -493,7 +508,7 @@ __device__ __forceinline__ bool trace_step8(L_& L, int2* s_stack, int2* l_stack,
     axis_terms8_xy(meta & 0xFFu, (meta >> 8) & 0xFFu, h0.x, h0.y, L.p.ox, L.p.oy, L.p.ix, L.p.iy, Sx, Sy, cnx, cny,
                    cfx, cfy);
     axis_terms8((meta >> 16) & 0xFFu, h0.z, L.p.oz, L.p.iz, Sz, cnz, cfz);
-    const float bound = __fmul_rn(L.best_t, kCullSlack);
+    const float bound = __fmaf_rn(L.best_t, kCullSlack, 0.0f);  // never -0 (see the masks below)
     // words: b0 = (lo.x[0-3], lo.x[4-7], hi.x[0-3], hi.x[4-7]), b1 the same for y, c0 for z
     const uint32_t lx0 = __float_as_uint(b0.x), lx1 = __float_as_uint(b0.y);
     const uint32_t hx0 = __float_as_uint(b0.z), hx1 = __float_as_uint(b0.w);
@@ -504,22 +519,27 @@ __device__ __forceinline__ bool trace_step8(L_& L, int2* s_stack, int2* l_stack,
     const uint32_t nx0 = sx ? hx0 : lx0, nx1 = sx ? hx1 : lx1, fx0 = sx ? lx0 : hx0, fx1 = sx ? lx1 : hx1;
     const uint32_t ny0 = sy ? hy0 : ly0, ny1 = sy ? hy1 : ly1, fy0 = sy ? ly0 : hy0, fy1 = sy ? ly1 : hy1;
     const uint32_t nz0 = sz ? hz0 : lz0, nz1 = sz ? hz1 : lz1, fz0 = sz ? lz0 : hz0, fz1 = sz ? lz1 : hz1;
-    uint32_t hm = 0;
+    // A child is missed when far - near is negative: the sign bits, two slots to a
+    // subtraction, are shifted into masks (against a compare, a select and an or
+    // a slot: 4 Mi closest-hit rays in 1 M triangles 3,373 -> 3,261 us, 1 M shadow rays
+    // 823 -> 800 us). The sign of a difference is that of the comparison; the one
+    // exception, -0 - (+0), needs far = -0, which neither a plane (a sum that
+    // cancels rounds to +0) nor `bound` can be.
+    uint32_t miss0 = 0, miss1 = 0;
 #pragma unroll
-    for (int b = 0; b < 4; ++b) {  // slots b and b + 4
+    for (int b = 3; b >= 0; --b) {  // slots b and b + 4
         const float2 tnx = plane_pair(nx0, nx1, b, Sx, cnx);
         const float2 tfx = plane_pair(fx0, fx1, b, Sx, cfx);
         const float2 tny = plane_pair(ny0, ny1, b, Sy, cny);
         const float2 tfy = plane_pair(fy0, fy1, b, Sy, cfy);
         const float2 tnz = plane_pair(nz0, nz1, b, Sz, cnz);
         const float2 tfz = plane_pair(fz0, fz1, b, Sz, cfz);
-        const float tnear0 = fmaxf(max3(tnx.x, tny.x, tnz.x), L.p.tmin);
-        const float tfar0 = fminf(min3(tfx.x, tfy.x, tfz.x), bound);
-        const float tnear1 = fmaxf(max3(tnx.y, tny.y, tnz.y), L.p.tmin);
-        const float tfar1 = fminf(min3(tfx.y, tfy.y, tfz.y), bound);
-        hm |= (tnear0 <= tfar0 ? 1u : 0u) << b;
-        hm |= (tnear1 <= tfar1 ? 1u : 0u) << (b + 4);
+        const float2 d = sub2(fminf(min3(tfx.x, tfy.x, tfz.x), bound), fminf(min3(tfx.y, tfy.y, tfz.y), bound),
+                              fmaxf(max3(tnx.x, tny.x, tnz.x), L.p.tmin), fmaxf(max3(tnx.y, tny.y, tnz.y), L.p.tmin));
+        miss0 = __funnelshift_l(__float_as_uint(d.x), miss0, 1);
+        miss1 = __funnelshift_l(__float_as_uint(d.y), miss1, 1);
     }
+    uint32_t hm = ~(miss0 | (miss1 << 4));
     hm &= valid;
     uint32_t thits = hm & ~imask;
     const uint32_t ihits = perm8[(oct << 8) | (hm & imask)];  // xor_permute8(hm & imask, oct)
