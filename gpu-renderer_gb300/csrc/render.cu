@@ -149,14 +149,12 @@ __device__ __forceinline__ Sample bsdf_sample(const Bsdf& b, V3 wo_w, float u0, 
     if (b.m->type == GR_MAT_DIFFUSE) {
         wi = cosine_hemisphere(u0, u1);
         if (wo.z < 0.0f) wi.z = -wi.z;
-        s.f = b.color * kInvPi * fabsf(wi.z);
         s.pdf = fabsf(wi.z) * kInvPi;
     } else if (b.m->type == GR_MAT_CONDUCTOR) {
         const V3 wh = ggx_sample_wh(wo, u0, u1, b.m->ax, b.m->ay);
         wi = reflect(wo, wh);
         if (!(wo.z * wi.z > 0.0f)) return s;
         s.pdf = mf_pdf_wh(b.m, wo, wh, b.compat);
-        s.f = mf_eval(b.m, b.color, wo, wi);
     } else if (b.m->type == GR_MAT_PLASTIC) {
         // pick a lobe with the first number and reuse its remainder (BSDF::sample, bsdf.h:109-120)
         const int lobe = min((int)floorf(u0 * 2.0f), 1);
@@ -169,7 +167,6 @@ __device__ __forceinline__ Sample bsdf_sample(const Bsdf& b, V3 wo_w, float u0, 
         }
         if (!(wo.z * wi.z > 0.0f)) return s;
         s.pdf = plastic_pdf(b, wo, wi);
-        s.f = plastic_eval(b, wo, wi);
     } else {
         const float F = fr_dielectric(wo.z, 1.0f, b.m->ior);
         if (u0 < F) {
@@ -272,6 +269,43 @@ __device__ __forceinline__ float tri_area(const SceneDev& sc, uint32_t prim) {
     return sqrtf(dot(c, c)) * 0.5f;
 }
 
+// The light records of a scene (LightDev), from its triangles: what every light
+// sample needs, computed once with the arithmetic shading would use.
+__global__ void k_lights(SceneDev sc, LightDev* __restrict__ out) {
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < sc.num_lights; i += gridDim.x * blockDim.x) {
+        const uint32_t prim = sc.lights[i], tm = sc.tri_mat[prim];
+        const float* t = sc.verts + 9ull * prim;
+        const DevMaterial* m = sc.mats + (tm & 0x3FFFFFFFu);
+        const V3 p0 = load3(t), p1 = load3(t + 3), p2 = load3(t + 6);
+        const V3 ng = normalize(cross(p0 - p2, p1 - p2));
+        LightDev l;
+        l.a = make_float4(p0.x, p0.y, p0.z, (1.0f / tri_area(sc, prim)) / (float)sc.num_lights);
+        l.b = make_float4(p1.x, p1.y, p1.z, __uint_as_float((tm & 0x80000000u) ? prim : 0xFFFFFFFFu));
+        l.c = make_float4(p2.x, p2.y, p2.z, m->er);
+        l.d = make_float4(ng.x, ng.y, ng.z, m->eg);
+        l.e = make_float4(m->eb, 0.0f, 0.0f, 0.0f);
+        out[i] = l;
+    }
+}
+
+// Point at barycentrics (u, v) of light `lid`: position, shading normal, the
+// density of picking it by area, and the light's radiance.
+__device__ __forceinline__ void light_point(const SceneDev& sc, uint32_t lid, float u, float v, V3& p, V3& ns,
+                                            float& pdf, V3& Le) {
+    const LightDev* l = sc.light_recs + lid;
+    const float4 a = __ldg(&l->a), b = __ldg(&l->b), c = __ldg(&l->c), d = __ldg(&l->d);
+    const float w = 1.0f - u - v;
+    p = v3(a.x, a.y, a.z) * w + v3(b.x, b.y, b.z) * u + v3(c.x, c.y, c.z) * v;
+    pdf = a.w;
+    ns = v3(d.x, d.y, d.z);
+    const uint32_t prim = __float_as_uint(b.w);
+    if (prim != 0xFFFFFFFFu) {
+        const float4 x = sc.normals[3ull * prim], y = sc.normals[3ull * prim + 1], z = sc.normals[3ull * prim + 2];
+        ns = normalize(v3(x.x, x.y, x.z) * w + v3(y.x, y.y, y.z) * u + v3(z.x, z.y, z.z) * v);
+    }
+    Le = v3(c.w, d.w, __ldg(&l->e.x));
+}
+
 __device__ __forceinline__ void add_acc(const Paths& ps, uint32_t pid, V3 L) {
     float4 a = ps.acc[pid];
     a.x += L.x;
@@ -292,6 +326,12 @@ __device__ __forceinline__ uint32_t find_job(const uint32_t* s_base, uint32_t nj
     return lo;
 }
 
+// x / J.npix for a path id x of the job (x < 2^31): a multiplication by the
+// rounded-up reciprocal that the host prepared (Granlund, Montgomery, PLDI 1994).
+__device__ __forceinline__ uint32_t div_npix(const JobDev& J, uint32_t x) {
+    return (uint32_t)(((uint64_t)x * J.npix_mul) >> J.npix_shift);
+}
+
 // ---- camera rays (generate_primary_rays_kernel, pathtracer_kernel.h:59-104) ------
 __global__ void __launch_bounds__(kShadeThreads) k_camera(Paths ps) {
     __shared__ uint32_t s_base[kMaxJobs + 1];
@@ -304,8 +344,9 @@ __global__ void __launch_bounds__(kShadeThreads) k_camera(Paths ps) {
         const uint32_t j = find_job(s_base, h.njobs, pid);
         const JobDev& J = ps.jobs[j];
         const uint32_t local = pid - J.path_base;
-        const uint32_t pixel = local % J.npix;
-        const uint32_t s = J.sample_base + local / J.npix;
+        const uint32_t sample = div_npix(J, local);
+        const uint32_t pixel = local - sample * J.npix;
+        const uint32_t s = J.sample_base + sample;
         const uint64_t inc = pcg_inc(pixel);
         uint64_t st = pcg_seed(J.seed + (uint64_t)s * kSampleStride, inc);
         const float j0 = pcg_float(st, inc), j1 = pcg_float(st, inc);
@@ -521,9 +562,9 @@ __global__ void __launch_bounds__(kShadeThreads, 4) k_shade(Paths ps, int b, Pcg
             const SceneDev& sc = J.sc;
             const bool compat = (J.flags & GR_RENDER_REFERENCE_COMPAT) != 0;
             const uint32_t local = pid - J.path_base;
-            const uint32_t pixel = local % J.npix;
-            const uint64_t inc = pcg_inc(pixel);
-            uint64_t st = pcg_seed(J.seed + (uint64_t)(J.sample_base + local / J.npix) * kSampleStride, inc);
+            const uint32_t sample = div_npix(J, local);
+            const uint64_t inc = pcg_inc(local - sample * J.npix);
+            uint64_t st = pcg_seed(J.seed + (uint64_t)(J.sample_base + sample) * kSampleStride, inc);
             st = st * jump.mul + inc * jump.add;
             const bool specular = (__float_as_uint(th.w) & kSpecularBit) != 0;
             V3 thr = v3(th.x, th.y, th.z);
@@ -560,12 +601,14 @@ __global__ void __launch_bounds__(kShadeThreads, 4) k_shade(Paths ps, int b, Pcg
                 }
             }
             if (alive && b < (int)J.max_depth) {
-                float s[8];
-#pragma unroll
-                for (int k = 0; k < 8; ++k) s[k] = pcg_float(st, inc);
                 if (prim < 0 || as_miss) {
                     if (sc.has_env) add(thr * env_radiance(sc, v3(r0.x, r0.y, r0.z), rd));
                 } else {
+                    // the bounce's eight numbers: light, light position (2), two unused, BSDF (2), one unused
+                    const float s0 = pcg_float(st, inc), s1 = pcg_float(st, inc), s2 = pcg_float(st, inc);
+                    pcg_next(st, inc);
+                    pcg_next(st, inc);
+                    const float s5 = pcg_float(st, inc), s6 = pcg_float(st, inc);
                     const uint32_t tm = sc.tri_mat[prim];
                     const DevMaterial* m = sc.mats + (tm & 0x3FFFFFFFu);
                     const Surf sf = surface(sc, (uint32_t)prim, hv.z, hv.w);
@@ -579,18 +622,17 @@ __global__ void __launch_bounds__(kShadeThreads, 4) k_shade(Paths ps, int b, Pcg
                     bs.compat = compat;
                     // next-event estimation with MIS
                     if (m->type != GR_MAT_DIELECTRIC && sc.num_lights > 0) {
-                        const uint32_t lid = min((uint32_t)(s[0] * (float)sc.num_lights), sc.num_lights - 1);
-                        const uint32_t lt = sc.lights[lid];
-                        const float a = sqrtf(s[1]);
-                        const Surf ls = surface(sc, lt, 1.0f - a, s[2] * a);
-                        float lpdf = (1.0f / tri_area(sc, lt)) / (float)sc.num_lights;
-                        V3 wi = ls.p - sf.p;
+                        const uint32_t lid = min((uint32_t)(s0 * (float)sc.num_lights), sc.num_lights - 1);
+                        const float a = sqrtf(s1);
+                        float lpdf;
+                        V3 lp, ln, Le;
+                        light_point(sc, lid, 1.0f - a, s2 * a, lp, ln, lpdf, Le);
+                        V3 wi = lp - sf.p;
                         const float d2 = dot(wi, wi);
                         wi = wi / sqrtf(d2);
-                        lpdf *= d2 / fabsf(dot(wi, ls.ns));
+                        lpdf *= d2 / fabsf(dot(wi, ln));
                         if (isinf(lpdf)) lpdf = 0.0f;
-                        const DevMaterial* lm = sc.mats + (sc.tri_mat[lt] & 0x3FFFFFFFu);
-                        const V3 Le = dot(-wi, ls.ns) > 0.0f ? v3(lm->er, lm->eg, lm->eb) : vs(0.0f);
+                        if (!(dot(-wi, ln) > 0.0f)) Le = vs(0.0f);
                         const V3 f = bsdf_eval(bs, wo, wi);
                         const float bp = bsdf_pdf(bs, wo, wi);
                         const float w = (lpdf * lpdf) / (lpdf * lpdf + bp * bp);
@@ -598,7 +640,7 @@ __global__ void __launch_bounds__(kShadeThreads, 4) k_shade(Paths ps, int b, Pcg
                             const V3 c = thr * Le * f * w / lpdf;
                             if (!black(c)) {
                                 const V3 so = sf.p - rd * 1.0e-4f;
-                                const V3 sd = ls.p - so;
+                                const V3 sd = lp - so;
                                 sh_r0 = make_float4(so.x, so.y, so.z, sd.x);
                                 sh_r1 = make_float4(sd.y, sd.z, 0.0f, r1.w);
                                 sh_c = make_float4(c.x, c.y, c.z, __uint_as_float(pid));
@@ -607,7 +649,7 @@ __global__ void __launch_bounds__(kShadeThreads, 4) k_shade(Paths ps, int b, Pcg
                         }
                     }
                     // BSDF sampling and scatter
-                    const Sample smp = bsdf_sample(bs, wo, s[5], s[6]);
+                    const Sample smp = bsdf_sample(bs, wo, s5, s6);
                     const V3 wgt = smp.pdf == 0.0f ? vs(0.0f) : thr * smp.f / smp.pdf;
                     if (!black(wgt)) {
                         new_r0 = make_float4(sf.p.x, sf.p.y, sf.p.z, smp.wi.x);
@@ -912,6 +954,10 @@ uint32_t pack_wave(std::vector<HostJob*>& jobs, uint32_t capacity, std::vector<J
         d.rr_depth = j->rr_depth;
         d.flags = j->flags;
         d.seed = j->seed;
+        uint32_t lg = 0;  // ceil(log2(npix))
+        while ((1ull << lg) < d.npix) ++lg;
+        d.npix_mul = (uint32_t)(((1ull << (31 + lg)) + d.npix - 1) / d.npix);
+        d.npix_shift = 31 + lg;
         out.push_back(d);
         paths += take * j->npix;
         pix += j->npix;
@@ -922,6 +968,12 @@ uint32_t pack_wave(std::vector<HostJob*>& jobs, uint32_t capacity, std::vector<J
     *total_pix = pix;
     *max_depth = depth;
     return (uint32_t)out.size();
+}
+
+cudaError_t light_records(const SceneDev& sc, LightDev* out, cudaStream_t s) {
+    if (sc.num_lights == 0) return cudaSuccess;
+    k_lights<<<std::min<uint32_t>((sc.num_lights + 127) / 128, 1024u), 128, 0, s>>>(sc, out);
+    return cudaGetLastError();
 }
 
 cudaError_t filter_rgba8(const double* fb, const uint32_t* fbc, uint32_t npix, uint32_t* out, cudaStream_t s) {

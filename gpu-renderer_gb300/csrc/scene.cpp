@@ -115,6 +115,7 @@ gr::SceneDev gr::scene_view(gr_scene* sc, int layout) {
     std::memcpy(d.env_c, sc->env_c, sizeof(d.env_c));
     d.mats = (const gr::DevMaterial*)sc->mats.p;
     d.lights = (const uint32_t*)sc->lights.p;
+    d.light_recs = (const gr::LightDev*)sc->light_recs.p;
     d.num_lights = sc->num_lights;
     d.num_tris = sc->num_tris;
     d.nodes = gr::layout_nodes(sc->bvh, layout);
@@ -303,6 +304,13 @@ gr_status gr_scene_create(gr_ctx* ctx, const gr_mesh* meshes, uint32_t num_meshe
     if (st != GR_OK) return cleanup(st);
     st = gr_bvh_build(sc->bvh, (const float*)sc->verts.p, (uint32_t)ntri, ctx->stream);
     if (st != GR_OK) return cleanup(st);
+    if (sc->num_lights) {
+        if ((e = sc->light_recs.ensure(sizeof(gr::LightDev) * (size_t)sc->num_lights)) != cudaSuccess)
+            return cleanup(cuda_fail(ctx, e, "scene upload alloc"));
+        if ((e = gr::light_records(gr::scene_view(sc, gr::kLayoutBvh2), (gr::LightDev*)sc->light_recs.p, ctx->stream)) !=
+            cudaSuccess)
+            return cleanup(cuda_fail(ctx, e, "light records"));
+    }
     if ((e = cudaStreamSynchronize(ctx->stream)) != cudaSuccess) return cleanup(cuda_fail(ctx, e, "bvh build"));
 
     sc->cam = gr::make_camera(*camera);

@@ -56,8 +56,8 @@ void mean_image(const double* sum, const uint32_t* cnt, uint32_t npix, float* ou
 extern "C" uint64_t gr_scene_device_bytes(const gr_scene* sc) {
     if (!sc) return 0;
     uint64_t b = sc->verts.bytes + sc->normals.bytes + sc->tri_mat.bytes + sc->mats.bytes + sc->lights.bytes +
-                 sc->uvs.bytes + sc->texels.bytes + sc->env_map.bytes +
-                 sc->fb.bytes + sc->fb_count.bytes;
+                 sc->light_recs.bytes + sc->uvs.bytes + sc->texels.bytes + sc->env_map.bytes + sc->fb.bytes +
+                 sc->fb_count.bytes;
     if (sc->bvh) {
         const gr::BvhBuffers& bb = sc->bvh->buf;
         b += bb.nodes.bytes + bb.nodes4.bytes + bb.nodes4q.bytes + bb.nodes8.bytes + bb.tris8.bytes + bb.tris.bytes +
