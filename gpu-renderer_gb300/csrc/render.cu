@@ -39,8 +39,8 @@ inline uint32_t draws_before(int b) { return b == 0 ? 2u : 9u * (uint32_t)b + 1u
 constexpr int kShadeThreads = 256;
 constexpr int kShadowBase = kMaxDepth + 1;  // shadow queue counters start here
 constexpr int kBinBase = 2 * kMaxDepth + 4;  // kShadeBins counters per bounce start here
-constexpr int kCntWords = (kBinBase + kShadeBins * (kMaxDepth + 1) + 1) & ~1;  // even: the work counters follow
-constexpr size_t kCounterBytes = sizeof(uint32_t) * kCntWords + sizeof(unsigned long long) * (kMaxDepth + 1);
+constexpr int kCntWords = kBinBase + kShadeBins * (kMaxDepth + 1);  // the work counters follow
+constexpr size_t kCounterBytes = sizeof(uint32_t) * kCntWords + sizeof(uint32_t) * (kMaxDepth + 1);
 
 __device__ __forceinline__ uint32_t lane_lt() {
     uint32_t m;
@@ -367,6 +367,9 @@ __global__ void __launch_bounds__(kShadeThreads) k_camera(Paths ps) {
 // ---- traversal over queues ----------------------------------------------------------
 // The BVH of a job's rays: nodes, triangles and root (the 8-wide root is node 0
 // of a scene with triangles, known without reading the BVH's header).
+// The job comes from the ray even when the wave has one job: kernels with the
+// job known beforehand, or its BVH kept in registers, were slower (glossy 54.8 and
+// 55.3 ms against 54.1).
 template <int LAYOUT>
 __device__ __forceinline__ uint32_t job_bvh(const JobDev* jobs, uint32_t j, const void*& nd, const Tri*& tr) {
     const SceneDev& sc = jobs[j].sc;
@@ -394,9 +397,7 @@ struct WaveSrc {
     float4* __restrict__ hits;
     float4* acc;
     const JobDev* jobs;
-    uint32_t nclosest;
-    uint64_t n;
-    bool one_job;  // the job is known before the ray has arrived
+    uint32_t nclosest, n;  // path state for 2^32 rays does not fit the GPU's memory, with room for the counter
     float tmin, tmax;
     __device__ __forceinline__ bool any(uint32_t i) const { return i >= nclosest; }
     __device__ __forceinline__ uint32_t load(uint32_t i, float4& r0, float4& r1, const void*& nd, const Tri*& tr) const {
@@ -404,7 +405,7 @@ struct WaveSrc {
         const float4* r = sh ? srays + 2ull * (i - nclosest) : rays + 2ull * i;
         r0 = __ldg(r);
         r1 = __ldg(r + 1);
-        const uint32_t root = job_bvh<LAYOUT>(jobs, one_job ? 0u : __float_as_uint(r1.w), nd, tr);
+        const uint32_t root = job_bvh<LAYOUT>(jobs, __float_as_uint(r1.w), nd, tr);
         r1.z = sh ? kShadowTmin : tmin;
         r1.w = sh ? kShadowTmax : tmax;
         return root;
@@ -432,9 +433,8 @@ __global__ void __launch_bounds__(trav::kMaxTraceThreads, 4) k_trace_wave(Paths 
     extern __shared__ int2 s_stack[];
     if (b > (int)ps.hdr->max_depth) return;
     const uint32_t nc = ps.cnt[b], ns = b ? ps.cnt[kShadowBase + b - 1] : 0u;
-    WaveSrc<LAYOUT> src{(b & 1) ? ps.ray[1] : ps.ray[0], ps.sray, ps.scon, ps.hit, ps.acc, ps.jobs, nc,
-                        (uint64_t)nc + ns, ps.hdr->njobs == 1, b == 0 ? kCameraTmin : kScatterTmin,
-                        b == 0 ? kCameraTmax : kScatterTmax};
+    WaveSrc<LAYOUT> src{(b & 1) ? ps.ray[1] : ps.ray[0], ps.sray, ps.scon, ps.hit, ps.acc, ps.jobs, nc, nc + ns,
+                        b == 0 ? kCameraTmin : kScatterTmin, b == 0 ? kCameraTmax : kScatterTmax};
     trav::traverse_loop<trav::kMixed, LAYOUT, SSTACK, trav::kRefillQueue>(
         src, trav::lanes_per_warp(src.n, gridDim.x * (blockDim.x / 32)), ps.work + b, &ps.hdr->err, s_stack);
 }
@@ -864,7 +864,7 @@ size_t path_layout(uint32_t cap, char* base, Paths* ps) {
     ps->sray = (float4*)take(32 * c);
     ps->scon = (float4*)take(16 * c);
     ps->cnt = (uint32_t*)take(kCounterBytes);  // counters and work counters, cleared as one
-    ps->work = (unsigned long long*)(ps->cnt + kCntWords);
+    ps->work = ps->cnt + kCntWords;
     ps->hdr = (WaveHeader*)take(sizeof(WaveHeader) + sizeof(JobDev) * kMaxJobs);
     ps->jobs = (JobDev*)(ps->hdr + 1);
     ps->capacity = cap;

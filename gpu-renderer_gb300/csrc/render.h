@@ -143,7 +143,7 @@ struct Paths {
     float4* sray;   // shadow rays, 2 per entry: (o.xyz, d.x), (d.y, d.z, 0, job bits); interval 0 .. 0.9999
     float4* scon;   // shadow contribution (rgb, path id bits)
     uint32_t* cnt;  // [0, kMaxDepth]: closest queue sizes; [kMaxDepth+1, ...]: shadow queue sizes
-    unsigned long long* work;  // dynamic-fetch counters, one per trace launch of a wave
+    uint32_t* work;  // dynamic-fetch counters, one per trace launch of a wave
     WaveHeader* hdr;
     JobDev* jobs;   // kMaxJobs entries
     uint32_t capacity;

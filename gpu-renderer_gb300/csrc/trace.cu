@@ -24,7 +24,7 @@ namespace gr {
 namespace {
 
 struct RaySrc {
-    using Index = uint64_t;
+    using Index = unsigned long long;
     const float4* __restrict__ rays;
     float4* __restrict__ hits;
     uint64_t n;
@@ -38,7 +38,7 @@ struct RaySrc {
         tr = tris;
         return root;
     }
-    __device__ __forceinline__ void finish(uint64_t i, const trav::Lane<uint64_t>& L) const {
+    __device__ __forceinline__ void finish(uint64_t i, const trav::Lane<Index>& L) const {
         hits[i] = L.best_prim == 0xFFFFFFFFu ? make_float4(L.p.tmax, __int_as_float(-1), 0.0f, 0.0f)
                                              : make_float4(L.best_t, __uint_as_float(L.best_prim), L.bu, L.bv);
     }

@@ -98,11 +98,35 @@ __device__ __forceinline__ bool slab(const RayW& p, float lox, float hix, float 
     return tnear <= __fmul_rn(tfar, kCullSlack);
 }
 
+// (a0 - b0, a1 - b1) in one packed subtraction, each rounded as a scalar one.
+__device__ __forceinline__ float2 sub2(float a0, float a1, float b0, float b1) {
+    float2 r;
+    asm("{\n\t"
+        ".reg .b64 a, b, r;\n\t"
+        "mov.b64 a, {%2, %3};\n\t"
+        "mov.b64 b, {%4, %5};\n\t"
+        "sub.rn.f32x2 r, a, b;\n\t"
+        "mov.b64 {%0, %1}, r;\n\t"
+        "}"
+        : "=f"(r.x), "=f"(r.y)
+        : "f"(a0), "f"(a1), "f"(b0), "f"(b1));
+    return r;
+}
+
+// PACKED: the x and y of a vertex are subtracted in one packed instruction (same
+// roundings). Faster in the 8-wide kernels, whose leaf loop is a third of their
+// instructions (batch of 8 scenes 8.31 -> 8.21 ms, Cornell box 1,105 -> 1,098 us), slower
+// in the binary one, which waits for its nodes (786 k camera rays 1,026 -> 1,031 us).
+template <bool PACKED>
 __device__ __forceinline__ bool tri_test(const RayW& p, const float4 a, const float4 b, const float4 c, float tbest,
                                          float& t, float& u, float& v) {
-    const float Ax0 = __fsub_rn(a.x, p.ox), Ay0 = __fsub_rn(a.y, p.oy), Az0 = __fsub_rn(a.z, p.oz);
-    const float Bx0 = __fsub_rn(b.x, p.ox), By0 = __fsub_rn(b.y, p.oy), Bz0 = __fsub_rn(b.z, p.oz);
-    const float Cx0 = __fsub_rn(c.x, p.ox), Cy0 = __fsub_rn(c.y, p.oy), Cz0 = __fsub_rn(c.z, p.oz);
+    const auto xy = [&](const float4 q) {
+        return PACKED ? sub2(q.x, q.y, p.ox, p.oy) : make_float2(__fsub_rn(q.x, p.ox), __fsub_rn(q.y, p.oy));
+    };
+    const float2 A0 = xy(a), B0 = xy(b), C0 = xy(c);
+    const float Ax0 = A0.x, Ay0 = A0.y, Az0 = __fsub_rn(a.z, p.oz);
+    const float Bx0 = B0.x, By0 = B0.y, Bz0 = __fsub_rn(b.z, p.oz);
+    const float Cx0 = C0.x, Cy0 = C0.y, Cz0 = __fsub_rn(c.z, p.oz);
     const float Akz = pick_axis(Ax0, Ay0, Az0, p.axes, 4), Bkz = pick_axis(Bx0, By0, Bz0, p.axes, 4), Ckz = pick_axis(Cx0, Cy0, Cz0, p.axes, 4);
     const float Ax = __fmaf_rn(-p.sx, Akz, pick_axis(Ax0, Ay0, Az0, p.axes, 0));
     const float Ay = __fmaf_rn(-p.sy, Akz, pick_axis(Ax0, Ay0, Az0, p.axes, 2));
@@ -173,12 +197,12 @@ __device__ __forceinline__ bool wants_any(const L_& L) {
 
 // Tests leaf triangle `c` (~sorted position); returns true when an any-hit
 // query is answered. Closest-hit ties at equal t go to the smaller prim id.
-template <int Q, class L_>
+template <int Q, bool PACKED = false, class L_>
 __device__ __forceinline__ bool leaf(L_& L, int32_t c) {
     const Tri* tr = L.tris + (uint32_t)(~c);
     const float4 a = __ldg(&tr->a), b = __ldg(&tr->b), cc = __ldg(&tr->c);
     float t, u, v;
-    if (!tri_test(L.p, a, b, cc, L.best_t, t, u, v)) return false;
+    if (!tri_test<PACKED>(L.p, a, b, cc, L.best_t, t, u, v)) return false;
     const uint32_t prim = __float_as_uint(a.w);
     const bool any = wants_any<Q>(L);
     if (any || t < L.best_t || prim < L.best_prim) {
@@ -396,21 +420,6 @@ __device__ __forceinline__ float2 plane_pair(uint32_t w0, uint32_t w1, int b, fl
     return t;
 }
 
-// (a0 - b0, a1 - b1) in one packed subtraction, each rounded as a scalar one.
-__device__ __forceinline__ float2 sub2(float a0, float a1, float b0, float b1) {
-    float2 r;
-    asm("{\n\t"
-        ".reg .b64 a, b, r;\n\t"
-        "mov.b64 a, {%2, %3};\n\t"
-        "mov.b64 b, {%4, %5};\n\t"
-        "sub.rn.f32x2 r, a, b;\n\t"
-        "mov.b64 {%0, %1}, r;\n\t"
-        "}"
-        : "=f"(r.x), "=f"(r.y)
-        : "f"(a0), "f"(a1), "f"(b0), "f"(b1));
-    return r;
-}
-
 // Per node and axis, with S = 2^e * (1/d) and C = (lo - o) * (1/d): the
 // plane scale S' = 2^15 * S (exact) and the near / far offsets C' -+ m with
 // C' = C - S' and m = |C| * 2^-20 + |S| * 2^-7. The roundings of C, C', the
@@ -492,7 +501,7 @@ __device__ __forceinline__ void stack_put(int i, int2 v, int2* s_stack, int2* l_
 
 // Leaf triangle `idx` of the layout's own triangle array.
 template <int Q, class L_>
-__device__ __forceinline__ bool leaf_at(L_& L, uint32_t idx) { return leaf<Q>(L, ~(int32_t)idx); }
+__device__ __forceinline__ bool leaf_at(L_& L, uint32_t idx) { return leaf<Q, true>(L, ~(int32_t)idx); }
 
 // One 8-wide node. A child plane is q * 2^e + lo, taken exactly; its ray
 // distance q * S + C, with S = 2^e / d (exact: a power-of-two scaling) and
@@ -637,7 +646,8 @@ __host__ __device__ inline uint32_t lanes_per_warp(uint64_t n, uint32_t warps) {
 }
 
 // Persistent dynamic-fetch loop. `Src` supplies the work:
-//   Index                                             integer type of a ray's index
+//   Index                                             integer type of a ray's index and of the work
+//                                                     counter (which ends up to a launch's lanes past n)
 //   n                                                 number of rays
 //   uint32_t load(Index i, float4& r0, float4& r1, const void*& nodes,
 //                 const Tri*& tris)                   ray i (reference Ray layout) and
@@ -652,8 +662,8 @@ __host__ __device__ inline uint32_t lanes_per_warp(uint64_t n, uint32_t warps) {
 // (traverse_smem). Every thread of the block calls it (the table is filled
 // behind a block barrier).
 template <int Q, int LAYOUT, int SSTACK, int REFILL, class Src>
-__device__ __forceinline__ void traverse_loop(Src& src, uint32_t lanes, unsigned long long* counter, uint32_t* err,
-                                              int2* s_stack) {
+__device__ __forceinline__ void traverse_loop(Src& src, uint32_t lanes, typename Src::Index* counter,
+                                              uint32_t* err, int2* s_stack) {
     int2 l_stack[kStackMax - SSTACK];
     // 8-wide layout: xor_permute8 as a table (octant x mask, 2 KB after the
     // short stacks), filled once per block
@@ -665,7 +675,7 @@ __device__ __forceinline__ void traverse_loop(Src& src, uint32_t lanes, unsigned
     const int lane = threadIdx.x & 31;
     const uint32_t ltmask = lanemask_lt();
     using Index = typename Src::Index;
-    const uint64_t n = src.n;
+    const Index n = src.n;
     // lanes past `lanes` stay idle; they count towards the threshold
     const int surplus = 32 - (int)lanes;
     const int refill = surplus + min(REFILL, (int)lanes);
@@ -678,28 +688,28 @@ __device__ __forceinline__ void traverse_loop(Src& src, uint32_t lanes, unsigned
         if (exhausted) {
             if (nidle == 32) break;  // a refill that found no rays leaves every lane idle
         } else if (nidle >= refill) {
-            unsigned long long base = 0;
+            Index base = 0;
             const int want = nidle - surplus;
-            if (lane == 0) base = atomicAdd(counter, (unsigned long long)want);
+            if (lane == 0) base = atomicAdd(counter, (Index)want);
             base = __shfl_sync(0xFFFFFFFFu, base, 0);
             if (base + want >= n) exhausted = true;
             if (!active && lane < (int)lanes) {
-                const uint64_t i = base + __popc(idle & ltmask);
+                const Index i = base + __popc(idle & ltmask);
                 if (i < n) {
                     float4 r0, r1;
-                    const uint32_t root = src.load((Index)i, r0, r1, L.nodes, L.tris);
+                    const uint32_t root = src.load(i, r0, r1, L.nodes, L.tris);
                     L.p = prepare(r0, r1);
                     L.best_t = L.p.tmax;
                     L.bu = 0.0f;
                     L.bv = 0.0f;
                     L.best_prim = 0xFFFFFFFFu;
-                    L.ray = (Index)i;
-                    if constexpr (Q == kMixed) L.any = src.any((Index)i);
+                    L.ray = i;
+                    if constexpr (Q == kMixed) L.any = src.any(i);
                     L.node = (LAYOUT == kLayoutBvh8Q8 && root != kNoNode) ? 0 : (int32_t)root;  // 8-wide root is node 0
                     L.sp = 0;
                     active = true;
                     if (root == kNoNode) {
-                        src.finish((Index)i, L);
+                        src.finish(i, L);
                         active = false;
                     }
                 }
