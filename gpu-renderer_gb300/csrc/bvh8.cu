@@ -402,7 +402,7 @@ __global__ void __launch_bounds__(kThreads8, 4) k8_build(Build8 B) {
             for (int w = 0; w < kWarps8; ++w) sum += s_warp[w];
             B.bsum[blockIdx.x] = sum;
         }
-        grid_barrier(B.sync, ++arrived * grid, B.err);
+        grid_sync(B.sync, ++arrived * grid, B.err);
         unsigned long long before = 0, total = 0;
         for (uint32_t j = threadIdx.x; j < grid; j += kThreads8) {
             const unsigned long long v = __ldcg(B.bsum + j);
@@ -458,7 +458,7 @@ __global__ void __launch_bounds__(kThreads8, 4) k8_build(Build8 B) {
             in_run += __popc(mi);
             leaf_run += __popc(ml);
         }
-        grid_barrier(B.sync, ++arrived * grid, B.err);
+        grid_sync(B.sync, ++arrived * grid, B.err);
         out_base = next_base;
         tri_cursor = (uint32_t)next_tri;
         n = (uint32_t)next_n;

@@ -14,15 +14,14 @@ __device__ __forceinline__ uint32_t ld_acquire(const uint32_t* p) {
 // Grid-wide barrier of a cooperative launch (every block resident): block
 // arrivals are counted on `ctr`, and the k-th barrier of the launch waits for
 // (k + 1) * gridDim.x arrivals, at most `limit` polls (then ERR_TIMEOUT).
-// The block barrier before the fence puts every thread's writes ahead of the
-// arrival; the block barrier after it puts the other blocks' writes ahead of
-// every thread's later reads (which go to L2: __ldcg).
+// The block barrier before the release puts every thread's writes ahead of the
+// arrival; the block barrier after the acquire puts the other blocks' writes
+// ahead of every thread's later reads (which go to L2: __ldcg).
 __device__ __forceinline__ void grid_barrier(uint32_t* ctr, uint32_t target, uint32_t* err,
                                              uint32_t limit = kSpinLimit) {
     __syncthreads();
     if (threadIdx.x == 0) {
-        __threadfence();
-        atomicAdd(ctr, 1u);
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(ctr) : "memory");
         uint32_t spins = 0;
         while (ld_acquire(ctr) < target) {
             if (++spins > limit) {
@@ -30,9 +29,15 @@ __device__ __forceinline__ void grid_barrier(uint32_t* ctr, uint32_t target, uin
                 break;
             }
         }
-        __threadfence();
     }
     __syncthreads();
+}
+
+// The same for a launch that may be a single block, which has nobody to wait for
+// (a barrier on its own counter took it 2 us).
+__device__ __forceinline__ void grid_sync(uint32_t* ctr, uint32_t target, uint32_t* err) {
+    if (gridDim.x == 1) __syncthreads();
+    else grid_barrier(ctr, target, err);
 }
 
 }  // namespace gr

@@ -332,7 +332,7 @@ __device__ __forceinline__ void sort_tile(const uint32_t* __restrict__ kin, cons
         // counts digit-major: column d holds digit d's count of every tile
         const uint32_t tiles = gridDim.x;
         if (threadIdx.x < 256) status[(size_t)threadIdx.x * tiles + tile] = cnt;
-        grid_barrier(sync_ctr, (barrier + 1) * gridDim.x, err);
+        grid_sync(sync_ctr, (barrier + 1) * gridDim.x, err);
         if (tiles <= kSumTiles) {
             // few tiles: each warp sums 16 digits' columns up to this tile,
             // 32 tiles per coalesced load
@@ -375,7 +375,7 @@ __device__ __forceinline__ void sort_tile(const uint32_t* __restrict__ kin, cons
                     carry += (uint32_t)sum;
                 }
             }
-            grid_barrier(sync_ctr, (barrier + 2) * gridDim.x, err);
+            grid_sync(sync_ctr, (barrier + 2) * gridDim.x, err);
             if (threadIdx.x < 256) {
                 s_dstart[threadIdx.x] = dstart;
                 s_gbase[threadIdx.x] = (uint32_t)(both >> 32) + __ldcg(status + (size_t)threadIdx.x * tiles + tile);
@@ -451,7 +451,7 @@ __global__ void __launch_bounds__(kOsThreads, 2) k_sort_coop(uint32_t* key_a, ui
         const bool even = (pass & 1) == 0;
         sort_tile<true>(even ? key_a : key_b, even ? val_a : val_b, even ? key_b : key_a, even ? val_b : val_a, n,
                         pass, hist, blockIdx.x, counts, sync_ctr, per_pass * pass, err, smem);
-        if (pass < 3) grid_barrier(sync_ctr, per_pass * (pass + 1) * gridDim.x, err);
+        if (pass < 3) grid_sync(sync_ctr, per_pass * (pass + 1) * gridDim.x, err);
     }
 }
 
@@ -514,14 +514,11 @@ __device__ __forceinline__ uint32_t run_depth(const uint32_t* __restrict__ code,
     return depth;
 }
 
-// Also clears the node counters of the bottom-up pass.
 __global__ void __launch_bounds__(kBlock) k_gaps(const uint32_t* __restrict__ code, uint32_t n,
-                                                 uint8_t* __restrict__ level, uint32_t* __restrict__ counters,
-                                                 uint32_t* __restrict__ err) {
+                                                 uint8_t* __restrict__ level, uint32_t* __restrict__ err) {
     for (uint32_t g = blockIdx.x * kBlock + threadIdx.x; g + 1 < n; g += gridDim.x * kBlock) {
         const uint32_t c0 = code[g], c1 = code[g + 1];
         level[g] = (uint8_t)(c0 != c1 ? (uint32_t)__clz(c0 ^ c1) : 32u + run_depth(code, n, g, err));
-        counters[g] = 0;
     }
 }
 
@@ -541,14 +538,14 @@ __device__ __forceinline__ Box3 get_child_box_l2(const Node* nd, int slot) {
     return b;
 }
 
-// Counter increment with acquire-release semantics at GPU scope: this thread's
-// earlier writes (its child box and link) are visible to the thread that sees
-// the incremented count, and the sibling's, written before its own increment,
+// Toggles bits of a word with acquire-release semantics at GPU scope: this
+// thread's earlier writes (its child box and link) are visible to the thread
+// that toggles the bit next, and the sibling's, written before its own toggle,
 // are visible to this thread's later reads. One ordered atomic in place of two
 // full fences around a relaxed one.
-__device__ __forceinline__ uint32_t atomic_add_acq_rel(uint32_t* p, uint32_t v) {
+__device__ __forceinline__ uint32_t atomic_xor_acq_rel(uint32_t* p, uint32_t v) {
     uint32_t old;
-    asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], %2;" : "=r"(old) : "l"(p), "r"(v) : "memory");
+    asm volatile("atom.acq_rel.gpu.global.xor.b32 %0, [%1], %2;" : "=r"(old) : "l"(p), "r"(v) : "memory");
     return old;
 }
 
@@ -574,14 +571,15 @@ struct Sub {
 // internal node and child slot the child's outer end and that end's outer-gap
 // level (far[2G] = the left child's first position and the level of the gap
 // before it, far[2G + 1] = the right child's last position and the level of
-// the gap after it), the node counters, and per chunk the subtree left to
-// attach across the chunk's left border.
+// the gap after it), a bit per gap that is set while exactly one child of its
+// node has arrived, and per chunk the subtree left to attach across the chunk's
+// left border.
 struct ClimbOut {
     Node* nodes;
     uint32_t* parent_leaf;
     unsigned long long* far;
     BvhMeta* meta;
-    uint32_t* counters;
+    uint32_t* arrived;
     Sub* pend;
     uint32_t* err;
 };
@@ -623,11 +621,11 @@ __device__ __forceinline__ void set_root(const ClimbOut& o, const Sub& s) {
     o.meta->root = (uint32_t)s.me;
 }
 
-// Climb from finished subtree `s` with GPU-scope counters: at each parent the
-// first arrival stops, the second unions its sibling's box and range and goes
-// on up. Two round trips a level: the counter, then the sibling's box and far
-// word (which carries the level the next step needs).
-__device__ __forceinline__ void climb_global(const ClimbOut& o, Sub s) {
+// Climbs from finished subtree `s`: at each parent the first arrival stops, the
+// second unions its sibling's box and range and goes on up. `arrive(G)` toggles
+// gap G's arrival bit and returns whether the sibling was there.
+template <class Arrive>
+__device__ __forceinline__ void climb(const ClimbOut& o, Sub s, Arrive arrive) {
     for (int guard = 0;; ++guard) {
         if (s.llo < 0 && s.lhi < 0) {
             set_root(o, s);
@@ -640,7 +638,7 @@ __device__ __forceinline__ void climb_global(const ClimbOut& o, Sub s) {
         const int slot = parent_slot(s);
         const uint32_t G = slot == 0 ? s.hi : s.lo - 1;
         attach(o, s, G, slot);
-        if (atomic_add_acq_rel(&o.counters[G], 1u) == 0) return;  // sibling not done yet
+        if (!arrive(G)) return;  // sibling not done yet
         box_union(s.box, get_child_box_l2(o.nodes + G, slot ^ 1));
         widen(s, slot, __ldcg(&o.far[2 * G + (slot ^ 1)]));
         s.me = (int32_t)G;
@@ -680,7 +678,7 @@ __device__ __forceinline__ uint32_t atomic_or_acq_rel_cta(uint32_t* p, uint32_t 
 // at most one subtree per chunk is left over: it goes to `pend`. After the
 // block barrier each thread writes, coalesced, its position's triangle and
 // leaf parent and its gap's node: the whole record if both children arrived,
-// else the one child's slot, far word and arrival count for part 2.
+// else the one child's slot and far word, and the gap's arrival bit, for part 2.
 __global__ void __launch_bounds__(kRefitChunk) k_climb_chunk(const float* __restrict__ verts, uint32_t n,
                                                              const uint32_t* __restrict__ prim,
                                                              const uint8_t* __restrict__ level, ClimbOut o,
@@ -766,8 +764,10 @@ __global__ void __launch_bounds__(kRefitChunk) k_climb_chunk(const float* __rest
             tris[p] = t;
             if (n > 1) o.parent_leaf[p] = leaf_parent;
         }
+        const uint32_t m = p + 1 < n ? s_mask[threadIdx.x] : 0u;
+        const uint32_t one = __ballot_sync(0xFFFFFFFFu, m == 1u || m == 2u);
+        if ((threadIdx.x & 31) == 0) o.arrived[p / 32] = one;
         if (p + 1 < n) {
-            const uint32_t m = s_mask[threadIdx.x];
             const int j = threadIdx.x;
             const float4* sb4 = reinterpret_cast<const float4*>(s_box[j]);
             const float4 u = sb4[0], w = sb4[1], z = sb4[2];
@@ -782,7 +782,6 @@ __global__ void __launch_bounds__(kRefitChunk) k_climb_chunk(const float* __rest
                 put_child_box(nd, slot, slot == 0 ? b0 : b1);
                 reinterpret_cast<int32_t*>(&nd->q3)[slot] = s_link[j][slot];
                 o.far[2 * p + slot] = s_far[j][slot];
-                o.counters[p] = 1;
             }
         }
         if (threadIdx.x == 0) o.pend[c] = s_pend;
@@ -791,27 +790,128 @@ __global__ void __launch_bounds__(kRefitChunk) k_climb_chunk(const float* __rest
 }
 
 // Bottom-up pass, part 2: one thread per chunk attaches the chunk's left-over
-// subtree (if any) across the chunk's left border and climbs with GPU-scope
-// counters. Part 1's writes are complete and visible (kernel boundary); every
-// node still open has exactly its missing arrivals left.
+// subtree (if any) across the chunk's left border and climbs. Part 1's writes are
+// complete and visible (kernel boundary); every node still open has exactly its
+// missing arrivals left. The root's chain is some 20 levels long and each level
+// waits for the one before, so the time is the level's latency.
+__device__ __forceinline__ bool load_sub(const Sub* ps, Sub& s) {
+    s.lo = ps->lo;
+    if (s.lo == 0) return false;  // nothing left over (a left-over range starts past 0)
+    s.me = ps->me;
+    s.hi = ps->hi;
+    s.llo = ps->llo;
+    s.lhi = ps->lhi;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        s.box.lo[k] = ps->box.lo[k];
+        s.box.hi[k] = ps->box.hi[k];
+    }
+    return true;
+}
+
+// In one block, for at most kBlockClimbChunks chunks. A thread that arrives first
+// at a node whose sibling part 1 did not finish leaves its subtree in shared
+// memory, in a table keyed by the gap (a thread waits at most once, so the table
+// never fills), and stops; the second arrival merges the two and writes the node's
+// whole record. Nothing of a level goes through L2 but the siblings that part 1
+// finished, about 1 us a level instead of 2. Build times, climbing over the whole
+// GPU against in one block: 300 triangles 54 / 48 us, 3,001 70 / 56, 10,000 85 / 70,
+// 100,003 99 / 93, 131,072 105 / 101; at 1 M the one block's throughput is the limit
+// (192 / 365 us with the siblings met through L2).
+constexpr uint32_t kBlockClimbChunks = 512;
+constexpr int kBlockClimbThreads = 1024;
+constexpr uint32_t kSpreadChunks = 64;
+constexpr uint32_t kClimbTable = 1024;  // power of two, twice the threads that can wait
+
+// Enters {G, id} in the table unless an entry for G is there; returns that
+// entry's id, or kNoNode when this one was entered (first arrival).
+__device__ __forceinline__ uint32_t meet(unsigned long long* table, uint32_t G, uint32_t id, uint32_t* err) {
+    constexpr unsigned long long kEmpty = ~0ull;
+    uint32_t h = (G * 2654435761u) >> 22;
+    for (uint32_t probe = 0; probe < kClimbTable; ++probe) {
+        const unsigned long long old = atomicCAS(&table[h], kEmpty, ((unsigned long long)G << 32) | id);
+        if (old == kEmpty) return kNoNode;
+        if ((uint32_t)(old >> 32) == G) return (uint32_t)old;
+        h = (h + 1) & (kClimbTable - 1);
+    }
+    atomicOr(err, ERR_RANGE);  // cannot happen
+    return kNoNode;
+}
+
+__global__ void __launch_bounds__(kBlockClimbThreads) k_climb_block(uint32_t chunks, ClimbOut o) {
+    __shared__ uint32_t s_bits[kBlockClimbChunks * kRefitChunk / 32];
+    __shared__ unsigned long long s_table[kClimbTable];
+    __shared__ Sub s_sub[kBlockClimbChunks];
+    static_assert(kClimbTable == 1u << 10, "the hash keeps ten bits");
+    for (uint32_t i = threadIdx.x; i < chunks * (kRefitChunk / 32); i += blockDim.x) s_bits[i] = o.arrived[i];
+    for (uint32_t i = threadIdx.x; i < kClimbTable; i += blockDim.x) s_table[i] = ~0ull;
+    __syncthreads();
+    Sub s;
+    // few chunks go to different warps, whose lanes would climb in step (3,001
+    // triangles 60 -> 56 us); many keep neighbours together (100 k: 93 against 97 us)
+    const uint32_t id = chunks <= kSpreadChunks
+                            ? (threadIdx.x & 31) * (kBlockClimbThreads / 32) + (threadIdx.x >> 5)
+                            : threadIdx.x;
+    if (id >= chunks || !load_sub(o.pend + id, s)) return;
+    for (int guard = 0;; ++guard) {  // s is finished, with its parent in its record, and is not the root
+        if (guard > 128) {
+            atomicOr(o.err, ERR_RANGE);
+            return;
+        }
+        const int slot = parent_slot(s);
+        const uint32_t G = slot == 0 ? s.hi : s.lo - 1;
+        Node* nd = o.nodes + G;
+        Sub t;  // the sibling, then the parent
+        if (s_bits[G / 32] >> (G & 31) & 1u) {  // finished by part 1
+            t.box = get_child_box_l2(nd, slot ^ 1);
+            t.me = __ldcg(reinterpret_cast<const int32_t*>(&nd->q3) + (slot ^ 1));
+            t.lo = t.hi = 0;
+            t.llo = t.lhi = -1;
+            // its outer end, as widen() would put it
+            widen(t, slot, __ldcg(&o.far[2 * G + (slot ^ 1)]));
+        } else {
+            s_sub[id] = s;
+            __threadfence_block();
+            const uint32_t other = meet(s_table, G, id, o.err);
+            if (other == kNoNode) return;  // sibling not done yet
+            __threadfence_block();
+            t = s_sub[other];
+        }
+        const Box3 sib = t.box;
+        const int32_t link = t.me;
+        t.me = (int32_t)G;
+        box_union(t.box, s.box);
+        if (slot == 0) {
+            t.lo = s.lo;
+            t.llo = s.llo;
+        } else {
+            t.hi = s.hi;
+            t.lhi = s.lhi;
+        }
+        const bool root = t.llo < 0 && t.lhi < 0;
+        const uint32_t parent = root ? kNoNode : (parent_slot(t) == 0 ? t.hi : t.lo - 1);
+        write_node(nd, slot == 0 ? s.box : sib, slot == 0 ? sib : s.box, slot == 0 ? s.me : link,
+                   slot == 0 ? link : s.me, parent);
+        if (root) {
+            o.meta->root = G;
+            return;
+        }
+        s = t;
+    }
+}
+
+// Over the whole GPU, ordered by GPU-scope atomics on the arrival bits in global
+// memory (2 us a level).
 constexpr int kUpThreads = 64;  // small blocks: the climbs spread over many SMs
 
 __global__ void __launch_bounds__(kUpThreads) k_climb_up(uint32_t chunks, ClimbOut o) {
     for (uint32_t c = blockIdx.x * kUpThreads + threadIdx.x; c < chunks; c += gridDim.x * kUpThreads) {
-        const Sub* ps = o.pend + c;
         Sub s;
-        s.lo = ps->lo;
-        if (s.lo == 0) continue;
-        s.me = ps->me;
-        s.hi = ps->hi;
-        s.llo = ps->llo;
-        s.lhi = ps->lhi;
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            s.box.lo[k] = ps->box.lo[k];
-            s.box.hi[k] = ps->box.hi[k];
-        }
-        climb_global(o, s);
+        if (!load_sub(o.pend + c, s)) continue;
+        climb(o, s, [&](uint32_t G) {
+            const uint32_t bit = 1u << (G & 31);
+            return (atomic_xor_acq_rel(o.arrived + G / 32, bit) & bit) != 0;
+        });
     }
 }
 
@@ -880,7 +980,7 @@ __global__ void __launch_bounds__(kBlock) k_export_ref(const Node* __restrict__ 
 size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 
 struct Scratch {
-    uint32_t *keys_alt, *vals_alt, *parent_leaf, *counters;
+    uint32_t *keys_alt, *vals_alt, *parent_leaf, *arrived;
     unsigned long long* far;
     Sub* pend;
     uint8_t* level;
@@ -905,10 +1005,11 @@ size_t scratch_layout(uint32_t n, char* base, Scratch* s) {
     s->vals_alt = (uint32_t*)take(w);
     s->parent_leaf = (uint32_t*)take(w);
     s->far = (unsigned long long*)take(16ull * n);
-    s->pend = (Sub*)take(sizeof(Sub) * (((uint64_t)n + kRefitChunk - 1) / kRefitChunk));
+    const uint64_t chunks = ((uint64_t)n + kRefitChunk - 1) / kRefitChunk;
+    s->pend = (Sub*)take(sizeof(Sub) * chunks);
     s->level = (uint8_t*)take(n);
     s->partial = (float*)take(sizeof(float) * 6 * kPartials);
-    s->counters = (uint32_t*)take(w);                            // cleared by k_gaps
+    s->arrived = (uint32_t*)take(kRefitChunk / 8 * chunks);     // written by k_climb_chunk
     s->os_status = (uint32_t*)take(4ull * os_tiles * 256 * 4);  // cleared by k_morton_hist
     // everything from here on is zeroed before each build
     const size_t zstart = off;
@@ -1033,11 +1134,14 @@ cudaError_t launch_build(const float* d_verts, uint32_t n, const Scratch& s, Nod
         }
     }
     // four passes: the sorted data is back in code/prim
-    k_gaps<<<grid, kBlock, 0, st>>>(code, n, s.level, s.counters, s.err);
+    k_gaps<<<grid, kBlock, 0, st>>>(code, n, s.level, s.err);
     const uint32_t chunks = (n + kRefitChunk - 1) / kRefitChunk;
-    const ClimbOut out{nodes, s.parent_leaf, s.far, meta, s.counters, s.pend, s.err};
+    const ClimbOut out{nodes, s.parent_leaf, s.far, meta, s.arrived, s.pend, s.err};
     k_climb_chunk<<<chunks, kRefitChunk, 0, st>>>(d_verts, n, prim, s.level, out, tris);
-    k_climb_up<<<(chunks + kUpThreads - 1) / kUpThreads, kUpThreads, 0, st>>>(chunks, out);
+    if (chunks > kBlockClimbChunks)
+        k_climb_up<<<(chunks + kUpThreads - 1) / kUpThreads, kUpThreads, 0, st>>>(chunks, out);
+    else if (chunks > 1)
+        k_climb_block<<<1, chunks <= kSpreadChunks ? kBlockClimbThreads : (int)(chunks + 31) / 32 * 32, 0, st>>>(chunks, out);
     // fold the build's error word into the header the host reads
     if ((e = cudaMemcpyAsync(&meta->err, s.err, 4, cudaMemcpyDeviceToDevice, st)) != cudaSuccess) return e;
     return cudaGetLastError();
@@ -1084,7 +1188,7 @@ cudaError_t lbvh_export_ref(const BvhBuffers& b, uint32_t n, uint32_t* d_ref_nod
 // every byte of device memory (and hands the plug-in only the buffers of a
 // call), and latency-critical loops in which a cudaMalloc / cudaFree would
 // synchronise the device. For them the build's scratch (sort buffers, split
-// levels, parent links, node counters, look-back words) lives in one
+// levels, parent links, arrival bits, look-back words) lives in one
 // file-scope device array, sized for kStaticMaxTriangles triangles; the caller
 // passes the input soup and every output buffer.
 //
@@ -1100,8 +1204,8 @@ constexpr uint32_t kStaticMaxTriangles = 1u << 17;  // 131,072 triangles
 
 constexpr size_t round256(size_t x) { return (x + 255) & ~size_t(255); }
 
-// Upper bound of scratch_layout(kStaticMaxTriangles): four per-triangle word
-// arrays (sort buffers, leaf parents, node counters), the two far words per
+// Upper bound of scratch_layout(kStaticMaxTriangles): three per-triangle word
+// arrays (sort buffers, leaf parents), the arrival bits, the two far words per
 // node, the left-over subtree per chunk, one level byte per gap, the centroid
 // partials, the histograms, the sort's look-back words (per tile of each
 // pass), tile counters and the error word, each rounded up to 256 bytes as
@@ -1109,8 +1213,9 @@ constexpr size_t round256(size_t x) { return (x + 255) & ~size_t(255); }
 constexpr size_t kStaticOsTiles = (kStaticMaxTriangles + kOsTile - 1) / kOsTile;
 constexpr size_t kStaticChunks = (kStaticMaxTriangles + kRefitChunk - 1) / kRefitChunk;
 constexpr size_t kStaticScratchBytes =
-    4 * round256((size_t)kStaticMaxTriangles * 4) + round256((size_t)kStaticMaxTriangles * 16) +
+    3 * round256((size_t)kStaticMaxTriangles * 4) + round256((size_t)kStaticMaxTriangles * 16) +
     round256(sizeof(Sub) * kStaticChunks) + round256(kStaticMaxTriangles) +
+    round256(kRefitChunk / 8 * kStaticChunks) +
     round256(sizeof(float) * 6 * kPartials) + 4096 + round256(4 * kStaticOsTiles * 256 * 4) + round256(16 * 4) +
     round256(4);
 
