@@ -5,7 +5,7 @@
 // :175-308). Differences by design:
 //   - persistent warps with dynamic refill: a fixed grid of warps pulls rays
 //     from a global counter, and a warp refills its idle lanes whenever at
-//     least kRefillRays of them have finished, until the queue is drained;
+//     least kRefill of them have finished, until the queue is drained;
 //   - child boxes live in the parent node and are fetched as 32-byte vector
 //     loads; all children are tested at once and the nearest is visited first;
 //   - a short per-thread stack in shared memory (8, 12 or 16 entries, chosen by
@@ -52,7 +52,8 @@ __global__ void __launch_bounds__(trav::kMaxTraceThreads, 4) k_trace(const void*
                                                                   uint32_t* err) {
     extern __shared__ int2 s_stack[];
     RaySrc src{rays, hits, n, nodes, tris, meta->root};
-    trav::traverse_loop<ANY ? trav::kAny : trav::kClosest, LAYOUT, SSTACK, trav::kRefillRays>(src, lanes, counter, err, s_stack);
+    constexpr int kRefill = LAYOUT == kLayoutBvh2 ? trav::kRefillRaysBvh2 : trav::kRefillRays;
+    trav::traverse_loop<ANY ? trav::kAny : trav::kClosest, LAYOUT, SSTACK, kRefill>(src, lanes, counter, err, s_stack);
 }
 
 template <bool ANY, int LAYOUT, int SSTACK>

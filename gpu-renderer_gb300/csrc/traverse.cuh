@@ -623,11 +623,21 @@ __device__ __forceinline__ bool trace_step(L_& L, int2* s_stack, int2* l_stack, 
 
 // A warp refills its idle lanes once at least REFILL of them are idle. The
 // ray-query kernels use 4 (a ray loads in two 16-byte reads; 2, 6 and 8
-// measured slower); the render's queue kernels use 12 (a queued ray also looks
-// up its job and scene; glossy 1024 x 768 x 64 spp: 72.4 ms at 8 and 12, 74.5 at
-// 4, 74.1 at 16).
+// measured slower), with binary nodes 8 (below); the render's queue kernels use 12
+// (a queued ray also looks up its job and scene; glossy 1024 x 768 x 64 spp: 72.4 ms
+// at 8 and 12, 74.5 at 4, 74.1 at 16).
 constexpr int kRefillRays = 4;
+constexpr int kRefillRaysBvh2 = 8;
 constexpr int kRefillQueue = 12;
+
+// Steps a lane takes between two looks at the warp's idle lanes. The look is a
+// warp vote, at which every lane waits for the slowest: a binary node's step is
+// short and waits for its node, so eight steps a vote are faster (786 k camera rays
+// in 300 k triangles 1,039 us at one step and refill at 4, 947 at four steps and 8,
+// 940 at eight steps; 2 Mi incoherent rays in 1 M triangles 2,820 -> 2,630 us; 1,021
+// rays 88 -> 76 us). An 8-wide node's step is long and issue bound, and there lanes
+// that idle until the vote cost more (4 Mi rays 3,257 us at one step, 3,381 at two).
+__host__ __device__ constexpr int steps_per_check(int layout) { return layout == kLayoutBvh2 ? 8 : 1; }
 
 // Lanes of a warp that take rays, for n rays on at most `warps` resident warps: a
 // launch that cannot give every lane of half the GPU's warps a ray spreads its
@@ -715,9 +725,19 @@ __device__ __forceinline__ void traverse_loop(Src& src, uint32_t lanes, typename
                 }
             }
         }
-        if (active && trace_step<Q, LAYOUT, SSTACK>(L, s_stack, l_stack, err, perm8)) {
-            src.finish(L.ray, L);
-            active = false;
+        if constexpr (steps_per_check(LAYOUT) == 1) {
+            if (active && trace_step<Q, LAYOUT, SSTACK>(L, s_stack, l_stack, err, perm8)) {
+                src.finish(L.ray, L);
+                active = false;
+            }
+        } else {
+#pragma unroll 1
+            for (int k = 0; k < steps_per_check(LAYOUT); ++k) {
+                if (active && trace_step<Q, LAYOUT, SSTACK>(L, s_stack, l_stack, err, perm8)) {
+                    src.finish(L.ray, L);
+                    active = false;
+                }
+            }
         }
     }
 }
