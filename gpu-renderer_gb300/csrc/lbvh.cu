@@ -14,6 +14,7 @@
 
 #include "gr_internal.h"
 #include "grid_sync.cuh"
+#include "launch.cuh"
 
 namespace gr {
 namespace {
@@ -128,6 +129,7 @@ __device__ __forceinline__ float block_bounds(float lo[3], float hi[3]) {
 __global__ void __launch_bounds__(kBlock) k_centroid(const float* __restrict__ verts, uint32_t n,
                                                      float* __restrict__ partial, uint32_t* __restrict__ done,
                                                      uint32_t* __restrict__ zero, uint32_t nzero, BvhMeta* meta) {
+    wait_for_previous();
     if (blockIdx.x == 0) {
         for (uint32_t i = threadIdx.x; i < nzero; i += kBlock) zero[i] = 0;
         if (threadIdx.x == 0) {
@@ -180,6 +182,7 @@ __global__ void __launch_bounds__(kBlock) k_morton_hist(const float* __restrict_
                                                         uint32_t* __restrict__ status, uint32_t nstatus) {
     __shared__ uint32_t s_hist[4 * 256];
     for (int i = threadIdx.x; i < 4 * 256; i += kBlock) s_hist[i] = 0;
+    wait_for_previous();
     for (uint32_t i = blockIdx.x * kBlock + threadIdx.x; i < nstatus; i += gridDim.x * kBlock) status[i] = 0;
     __syncthreads();
     float blo[3], bhi[3];
@@ -442,6 +445,7 @@ __global__ void __launch_bounds__(kOsThreads, 2) k_onesweep(const uint32_t* __re
                                                          uint32_t* __restrict__ err) {
     extern __shared__ uint32_t smem[];
     __shared__ uint32_t s_tile;
+    wait_for_previous();
     if (threadIdx.x == 0) s_tile = atomicAdd(tile_ctr + pass, 1u);
     __syncthreads();
     sort_tile<false>(kin, vin, kout, vout, n, pass, hist, s_tile, status, nullptr, 0, err, smem);
@@ -529,6 +533,7 @@ __device__ __forceinline__ uint32_t run_depth(const uint32_t* __restrict__ code,
 __global__ void __launch_bounds__(kBlock) k_gaps(const uint32_t* __restrict__ code, uint32_t n,
                                                  uint8_t* __restrict__ level, uint32_t* __restrict__ done,
                                                  uint32_t* __restrict__ err) {
+    wait_for_previous();
     // zero already, unless builds sharing the scratch overlapped: a build leaves it so for the next
     if (blockIdx.x == 0 && threadIdx.x == 0) *done = 0;
     for (uint32_t g = blockIdx.x * kBlock + threadIdx.x; g + 1 < n; g += gridDim.x * kBlock) {
@@ -704,6 +709,7 @@ __global__ void __launch_bounds__(kRefitChunk) k_climb_chunk(const float* __rest
     __shared__ unsigned long long s_far[kRefitChunk][2];
     __shared__ int32_t s_link[kRefitChunk][2];
     __shared__ Sub s_pend;
+    wait_for_previous();
     const uint32_t chunks = (n + kRefitChunk - 1) / kRefitChunk;
     for (uint32_t c = blockIdx.x; c < chunks; c += gridDim.x) {  // block-uniform
         const uint32_t base = c * kRefitChunk;
@@ -858,8 +864,9 @@ __global__ void __launch_bounds__(kBlockClimbThreads) k_climb_block(uint32_t chu
     __shared__ unsigned long long s_table[kClimbTable];
     __shared__ Sub s_sub[kBlockClimbChunks];
     static_assert(kClimbTable == 1u << 10, "the hash keeps ten bits");
-    for (uint32_t i = threadIdx.x; i < chunks * (kRefitChunk / 32); i += blockDim.x) s_bits[i] = o.arrived[i];
     for (uint32_t i = threadIdx.x; i < kClimbTable; i += blockDim.x) s_table[i] = ~0ull;
+    wait_for_previous();
+    for (uint32_t i = threadIdx.x; i < chunks * (kRefitChunk / 32); i += blockDim.x) s_bits[i] = o.arrived[i];
     __syncthreads();
     Sub s;
     // few chunks go to different warps, whose lanes would climb in step (3,001
@@ -920,6 +927,7 @@ __global__ void __launch_bounds__(kBlockClimbThreads) k_climb_block(uint32_t chu
 constexpr int kUpThreads = 64;  // small blocks: the climbs spread over many SMs
 
 __global__ void __launch_bounds__(kUpThreads) k_climb_up(uint32_t chunks, ClimbOut o) {
+    wait_for_previous();
     for (uint32_t c = blockIdx.x * kUpThreads + threadIdx.x; c < chunks; c += gridDim.x * kUpThreads) {
         Sub s;
         if (!load_sub(o.pend + c, s)) continue;
@@ -1095,6 +1103,14 @@ cudaError_t sort_coop_capacity(int num_sms, int* tiles) {
     return cudaSuccess;
 }
 
+// Builds of up to this many triangles overlap the launches of their kernels (launch.cuh).
+constexpr uint32_t kOverlapTriangles = 1u << 18;
+
+#define LB_TRY(call)                                \
+    do {                                            \
+        if ((e = (call)) != cudaSuccess) return e; \
+    } while (0)
+
 // The build's launch sequence over laid-out scratch `s` (scratch_layout): the
 // one both the allocating build and the no-allocation build run. Centroid bounds
 // (and clearing), Morton codes and histograms, the sort (the sorted codes and
@@ -1103,13 +1119,14 @@ cudaError_t sort_coop_capacity(int num_sms, int* tiles) {
 cudaError_t launch_build(const float* d_verts, uint32_t n, const Scratch& s, Node* nodes, Tri* tris, uint32_t* code,
                          uint32_t* prim, BvhMeta* meta, int num_sms, cudaStream_t st) {
     cudaError_t e;
+    const bool small = n <= kOverlapTriangles;
     const int grid = (int)std::min<uint64_t>(((uint64_t)n + kBlock - 1) / kBlock, (uint64_t)num_sms * 8);
     const int parts = std::min(grid, kPartials);
-    k_centroid<<<parts, kBlock, 0, st>>>(d_verts, n, s.partial, s.done, s.hist, s.zero_words, meta);
+    LB_TRY(launch_after(small, k_centroid, parts, kBlock, 0, st, d_verts, n, s.partial, s.done, s.hist, s.zero_words, meta));
     uint32_t* err = &meta->err;
     const uint32_t os_tiles = (n + kOsTile - 1) / kOsTile;
-    k_morton_hist<<<std::min(grid, num_sms * 2), kBlock, 0, st>>>(d_verts, n, meta, code, prim, s.hist, s.os_status,
-                                                                  4 * os_tiles * 256);
+    LB_TRY(launch_after(small, k_morton_hist, std::min(grid, num_sms * 2), kBlock, 0, st, d_verts, n, meta, code, prim, s.hist,
+                        s.os_status, 4 * os_tiles * 256));
     if ((e = cudaFuncSetAttribute(k_onesweep, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kOsSmem)) !=
         cudaSuccess)
         return e;
@@ -1138,22 +1155,23 @@ cudaError_t launch_build(const float* d_verts, uint32_t n, const Scratch& s, Nod
         uint32_t* kout = s.keys_alt;
         uint32_t* vout = s.vals_alt;
         for (int pass = 0; pass < 4; ++pass) {
-            k_onesweep<<<os_tiles, kOsThreads, kOsSmem, st>>>(kin, vin, kout, vout, n, pass, s.hist,
-                                                              s.os_status + (size_t)pass * os_tiles * 256,
-                                                              s.tile_ctr, err);
+            LB_TRY(launch_after(small, k_onesweep, os_tiles, kOsThreads, kOsSmem, st, kin, vin, kout, vout, n, pass, s.hist,
+                                s.os_status + (size_t)pass * os_tiles * 256, s.tile_ctr, err));
             std::swap(kin, kout);
             std::swap(vin, vout);
         }
     }
     // four passes: the sorted data is back in code/prim
-    k_gaps<<<grid, kBlock, 0, st>>>(code, n, s.level, s.done, err);
+    LB_TRY(launch_after(small, k_gaps, grid, kBlock, 0, st, code, n, s.level, s.done, err));
     const uint32_t chunks = (n + kRefitChunk - 1) / kRefitChunk;
     const ClimbOut out{nodes, s.parent_leaf, s.far, meta, s.arrived, s.pend, err};
-    k_climb_chunk<<<chunks, kRefitChunk, 0, st>>>(d_verts, n, prim, s.level, out, tris);
-    if (chunks > kBlockClimbChunks)
-        k_climb_up<<<(chunks + kUpThreads - 1) / kUpThreads, kUpThreads, 0, st>>>(chunks, out);
-    else if (chunks > 1)
-        k_climb_block<<<1, chunks <= kSpreadChunks ? kBlockClimbThreads : (int)(chunks + 31) / 32 * 32, 0, st>>>(chunks, out);
+    LB_TRY(launch_after(small, k_climb_chunk, chunks, kRefitChunk, 0, st, d_verts, n, prim, s.level, out, tris));
+    if (chunks > kBlockClimbChunks) {
+        LB_TRY(launch_after(small, k_climb_up, (chunks + kUpThreads - 1) / kUpThreads, kUpThreads, 0, st, chunks, out));
+    } else if (chunks > 1) {
+        const uint32_t threads = chunks <= kSpreadChunks ? kBlockClimbThreads : (chunks + 31) / 32 * 32;
+        LB_TRY(launch_after(small, k_climb_block, 1, threads, 0, st, chunks, out));
+    }
     return cudaGetLastError();
 }
 

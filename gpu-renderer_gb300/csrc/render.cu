@@ -19,6 +19,7 @@
 #include <cstddef>
 #include <cstring>
 
+#include "launch.cuh"
 #include "render.h"
 #include "shading.cuh"
 #include "traverse.cuh"
@@ -335,6 +336,7 @@ __device__ __forceinline__ uint32_t div_npix(const JobDev& J, uint32_t x) {
 // ---- camera rays (generate_primary_rays_kernel, pathtracer_kernel.h:59-104) ------
 __global__ void __launch_bounds__(kShadeThreads) k_camera(Paths ps) {
     __shared__ uint32_t s_base[kMaxJobs + 1];
+    wait_for_previous();
     const WaveHeader h = *ps.hdr;
     for (uint32_t j = threadIdx.x; j < h.njobs; j += blockDim.x) s_base[j] = ps.jobs[j].path_base;
     if (threadIdx.x == 0) s_base[h.njobs] = h.total_paths;
@@ -431,6 +433,7 @@ struct WaveSrc {
 template <int LAYOUT, int SSTACK>
 __global__ void __launch_bounds__(trav::kMaxTraceThreads, 4) k_trace_wave(Paths ps, int b) {
     extern __shared__ int2 s_stack[];
+    wait_for_previous();
     if (b > (int)ps.hdr->max_depth) return;
     const uint32_t nc = ps.cnt[b], ns = b ? ps.cnt[kShadowBase + b - 1] : 0u;
     WaveSrc<LAYOUT> src{(b & 1) ? ps.ray[1] : ps.ray[0], ps.sray, ps.scon, ps.hit, ps.acc, ps.jobs, nc, nc + ns,
@@ -458,6 +461,7 @@ __device__ __forceinline__ uint32_t* bin_entry(const Paths& ps, int k, uint32_t 
 }
 
 __global__ void __launch_bounds__(kShadeThreads) k_bin(Paths ps, int b) {
+    wait_for_previous();
     if (b > (int)ps.hdr->max_depth) return;
     const uint32_t n = ps.cnt[b];
     const float4* rays = (b & 1) ? ps.ray[1] : ps.ray[0];
@@ -522,6 +526,7 @@ __global__ void __launch_bounds__(kShadeThreads) k_bin(Paths ps, int b) {
 // queue itself (waves whose scenes use one material type).
 template <bool BINNED>
 __global__ void __launch_bounds__(kShadeThreads, 4) k_shade(Paths ps, int b, PcgJump jump) {
+    wait_for_previous();
     if (b > (int)ps.hdr->max_depth) return;
     __shared__ uint32_t s_first[kShadeBins + 1];
     if (BINNED) {
@@ -690,6 +695,7 @@ __device__ __forceinline__ double widen(float f) {
 // ---- resolve: paths -> pixels in sample order ------------------------------------------
 __global__ void __launch_bounds__(kShadeThreads) k_resolve(Paths ps) {
     __shared__ uint32_t s_base[kMaxJobs + 1];
+    wait_for_previous();
     const WaveHeader h = *ps.hdr;
     for (uint32_t j = threadIdx.x; j < h.njobs; j += blockDim.x) s_base[j] = ps.jobs[j].pix_base;
     if (threadIdx.x == 0) s_base[h.njobs] = h.total_pix;
@@ -780,45 +786,46 @@ __global__ void __launch_bounds__(kShadeThreads) k_mean_rgb(const double* __rest
     }
 }
 
+// Waves of up to this many paths overlap the launches of their kernels (launch.cuh).
+constexpr uint32_t kOverlapPaths = 1u << 16;
+
 // One wave: clear counters, camera rays, depth_steps x (trace, shade)
 // (steps past the wave's max_depth return at once), resolve (which adds the ray counts up).
 template <int LAYOUT, int SSTACK>
 cudaError_t issue_wave_l(const Paths& ps, uint32_t depth_steps, int tgrid, int tblock, int sgrid, bool bin,
-                         cudaStream_t s) {
+                         bool small, cudaStream_t s) {
     const size_t smem = trav::traverse_smem(LAYOUT, SSTACK, tblock);
     cudaError_t e;
     if ((e = cudaMemsetAsync(ps.cnt, 0, kCounterBytes, s)) != cudaSuccess) return e;
-    k_camera<<<2 * sgrid, kShadeThreads, 0, s>>>(ps);
+    if ((e = launch_after(small, k_camera, 2 * sgrid, kShadeThreads, 0, s, ps)) != cudaSuccess) return e;
     for (int b = 0; b <= (int)depth_steps; ++b) {
-        k_trace_wave<LAYOUT, SSTACK><<<tgrid, tblock, smem, s>>>(ps, b);
+        if ((e = launch_after(small, k_trace_wave<LAYOUT, SSTACK>, tgrid, tblock, smem, s, ps, b)) != cudaSuccess) return e;
         const PcgJump jump = pcg_jump(draws_before(b));
-        if (bin) {
-            k_bin<<<2 * sgrid, kShadeThreads, 0, s>>>(ps, b);
-            k_shade<true><<<sgrid, kShadeThreads, 0, s>>>(ps, b, jump);
-        } else {
-            k_shade<false><<<sgrid, kShadeThreads, 0, s>>>(ps, b, jump);
-        }
+        if (bin && (e = launch_after(small, k_bin, 2 * sgrid, kShadeThreads, 0, s, ps, b)) != cudaSuccess) return e;
+        e = bin ? launch_after(small, k_shade<true>, sgrid, kShadeThreads, 0, s, ps, b, jump)
+                : launch_after(small, k_shade<false>, sgrid, kShadeThreads, 0, s, ps, b, jump);
+        if (e != cudaSuccess) return e;
     }
-    k_resolve<<<2 * sgrid, kShadeThreads, 0, s>>>(ps);
+    if ((e = launch_after(small, k_resolve, 2 * sgrid, kShadeThreads, 0, s, ps)) != cudaSuccess) return e;
     return cudaGetLastError();
 }
 
 template <int LAYOUT>
 cudaError_t issue_wave_s(const Paths& ps, uint32_t steps, int tgrid, const TraceTuning& t, int sgrid, bool bin,
-                         cudaStream_t s) {
-    if (t.sstack == 8) return issue_wave_l<LAYOUT, 8>(ps, steps, tgrid, t.block, sgrid, bin, s);
-    if (t.sstack == 16) return issue_wave_l<LAYOUT, 16>(ps, steps, tgrid, t.block, sgrid, bin, s);
-    return issue_wave_l<LAYOUT, 12>(ps, steps, tgrid, t.block, sgrid, bin, s);
+                         bool small, cudaStream_t s) {
+    if (t.sstack == 8) return issue_wave_l<LAYOUT, 8>(ps, steps, tgrid, t.block, sgrid, bin, small, s);
+    if (t.sstack == 16) return issue_wave_l<LAYOUT, 16>(ps, steps, tgrid, t.block, sgrid, bin, small, s);
+    return issue_wave_l<LAYOUT, 12>(ps, steps, tgrid, t.block, sgrid, bin, small, s);
 }
 
 // bin: group the paths by material before shading (waves whose scenes mix
 // material types).
-cudaError_t issue_wave(const Paths& ps, uint32_t steps, int tgrid, int sgrid, bool bin, cudaStream_t s,
-                       const TraceTuning& t) {
-    if (t.layout == kLayoutBvh4) return issue_wave_s<kLayoutBvh4>(ps, steps, tgrid, t, sgrid, bin, s);
-    if (t.layout == kLayoutBvh4Q8) return issue_wave_s<kLayoutBvh4Q8>(ps, steps, tgrid, t, sgrid, bin, s);
-    if (t.layout == kLayoutBvh8Q8) return issue_wave_s<kLayoutBvh8Q8>(ps, steps, tgrid, t, sgrid, bin, s);
-    return issue_wave_s<kLayoutBvh2>(ps, steps, tgrid, t, sgrid, bin, s);
+cudaError_t issue_wave(const Paths& ps, uint32_t steps, int tgrid, int sgrid, bool bin, bool small,
+                       cudaStream_t s, const TraceTuning& t) {
+    if (t.layout == kLayoutBvh4) return issue_wave_s<kLayoutBvh4>(ps, steps, tgrid, t, sgrid, bin, small, s);
+    if (t.layout == kLayoutBvh4Q8) return issue_wave_s<kLayoutBvh4Q8>(ps, steps, tgrid, t, sgrid, bin, small, s);
+    if (t.layout == kLayoutBvh8Q8) return issue_wave_s<kLayoutBvh8Q8>(ps, steps, tgrid, t, sgrid, bin, small, s);
+    return issue_wave_s<kLayoutBvh2>(ps, steps, tgrid, t, sgrid, bin, small, s);
 }
 
 // Resident blocks per SM of the wave's traversal kernel for a configuration.
@@ -1029,10 +1036,11 @@ cudaError_t run_wave(WavePool& pool, const JobDev* h_jobs, uint32_t njobs, uint3
     uint32_t types = 0;
     for (uint32_t j = 0; j < njobs; ++j) types |= h_jobs[j].sc.mat_types;
     const bool bin = __builtin_popcount(types) >= 2;
-    if (!use_graph) return issue_wave(ps, max_depth, tgrid, sgrid, bin, s, tune);
+    const bool small = total_paths <= kOverlapPaths;
+    if (!use_graph) return issue_wave(ps, max_depth, tgrid, sgrid, bin, small, s, tune);
     uint64_t key = 0x51ED270B27A3C1F5ull;
     const uint64_t words[] = {(uint64_t)(uintptr_t)ps.ray[0], ps.capacity, steps, (uint64_t)tgrid, (uint64_t)sgrid,
-                              (uint64_t)tune.layout, (uint64_t)tune.block, (uint64_t)tune.sstack, (uint64_t)bin};
+                              (uint64_t)tune.layout, (uint64_t)tune.block, (uint64_t)tune.sstack, (uint64_t)bin, (uint64_t)small};
     for (uint64_t w : words) key = mix64(key, w);
     int hit = -1;
     for (int i = 0; i < WavePool::kGraphs; ++i)
@@ -1050,7 +1058,7 @@ cudaError_t run_wave(WavePool& pool, const JobDev* h_jobs, uint32_t njobs, uint3
     if (!g.exec) {
         cudaGraph_t graph = nullptr;
         if ((e = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal)) != cudaSuccess) return e;
-        const cudaError_t ei = issue_wave(ps, steps, tgrid, sgrid, bin, s, tune);
+        const cudaError_t ei = issue_wave(ps, steps, tgrid, sgrid, bin, small, s, tune);
         e = cudaStreamEndCapture(s, &graph);
         if (ei != cudaSuccess) {
             if (graph) cudaGraphDestroy(graph);
