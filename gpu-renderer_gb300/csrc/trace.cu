@@ -72,7 +72,8 @@ cudaError_t launch(const BvhDevice& bvh, const void* nodes, int block, const flo
     const uint32_t lanes = trav::lanes_per_warp(n, warps);
     const uint64_t warps_needed = (n + lanes - 1) / lanes;
     const uint64_t blocks_needed = (warps_needed + block / 32 - 1) / (block / 32);
-    const int grid = (int)std::min<uint64_t>((uint64_t)num_sms * occ[bi], blocks_needed);
+    const uint64_t resident = (uint64_t)num_sms * occ[bi] * trav::resident_eighths(LAYOUT, n, warps) / 8;
+    const int grid = (int)std::min<uint64_t>(std::max<uint64_t>(resident, 1), blocks_needed);
     k_trace<ANY, LAYOUT, SSTACK><<<grid, block, smem, s>>>(nodes, bvh.tris, bvh.meta, r, n, lanes, h, counter, err);
     return cudaGetLastError();
 }

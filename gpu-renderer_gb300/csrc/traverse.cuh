@@ -655,6 +655,19 @@ __host__ __device__ inline uint32_t lanes_per_warp(uint64_t n, uint32_t warps) {
     return per >= 32 ? 32u : (per < 1 ? 1u : (uint32_t)per);
 }
 
+// Eighths of the resident warps that an 8-wide ray query of n rays uses. With few
+// rays per lane much of a launch is its tail, where every warp is still there for
+// its last rays, and fewer warps run a ray's steps faster: incoherent rays in 1 M
+// triangles, all warps against the best share (us): 100 k rays 269 / 248 (1/2), 155 k
+// 349 / 298 (5/8), 200 k 374 / 341 (5/8), 262 k 416 / 391 (3/4), 400 k 508 / 500 (7/8),
+// 600 k 652 / 653, 1 M 926 / 940 (7/8). Binary nodes, which wait for memory, gain 3 % at
+// most and use all; so do a render's waves, where it changed nothing.
+inline uint32_t resident_eighths(int layout, uint64_t n, uint32_t warps) {
+    if (layout != kLayoutBvh8Q8) return 8;
+    const uint64_t lanes = 32ull * warps, tenths = n > 100 * lanes ? 1000 : 10 * n / lanes;  // of rays per lane
+    return tenths < 8 ? 4 : (tenths < 13 ? 5 : (tenths < 22 ? 6 : (tenths < 32 ? 7 : 8)));
+}
+
 // Persistent dynamic-fetch loop. `Src` supplies the work:
 //   Index                                             integer type of a ray's index and of the work
 //                                                     counter (which ends up to a launch's lanes past n)

@@ -26,3 +26,19 @@ def test_hits_match_oracle_at_every_fill(ctx, oracle, layout, block):
         np.testing.assert_array_equal(b.trace_host(sh[:n], any_hit=True).view(np.uint32), want_any[:n].view(np.uint32),
                                       err_msg=str(n))
     b.close()
+
+
+@pytest.mark.parametrize("block", [64, 128, 256])
+def test_hits_match_oracle_at_every_share_of_the_warps(ctx, oracle, block):
+    """8-wide ray queries use between half and all of the resident warps: counts on
+    both sides of each change (rays per resident lane 0.8, 1.3, 2.2, 3.2)."""
+    v = sc.triangle_soup(3000, seed_salt=81)
+    b = gr.BVH(ctx)
+    b.build_host(v)
+    b.set_tuning(gr.LAYOUT_BVH8_Q8, block, 12)
+    ob = oracle.lbvh(v)
+    inc = sc.incoherent_rays(520000, seed_salt=82)
+    want = oracle.trace(ob, inc).view(np.uint32)
+    for n in (77824, 110000, 124517, 124519, 202342, 202343, 342425, 342426, 498073, 498074, 520000):
+        np.testing.assert_array_equal(b.trace_host(inc[:n]).view(np.uint32), want[:n], err_msg=str(n))
+    b.close()
