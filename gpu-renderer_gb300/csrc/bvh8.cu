@@ -36,6 +36,7 @@ constexpr int kLanesPerNode = 8;                  // lanes collapsing one 8-wide
 constexpr int kNodesPerWarp = 32 / kLanesPerNode;
 constexpr int32_t kEmptySlot = INT32_MIN;
 constexpr uint32_t kMaxLevels8 = 72;
+constexpr uint32_t kAloneNodes = kWarps8 * kNodesPerWarp;  // levels that one block takes in one step
 
 // 8-wide planes: plane(q) = q * 2^e + lo, taken EXACTLY (the traversal
 // measures it as fma(q, 2^e / d, (lo - o) / d) with error margins, never
@@ -129,6 +130,11 @@ struct Size8 {
     uint32_t nodes, tris, overflow, pad;
 };
 
+// Where the build stands between two levels.
+struct Level8 {
+    uint32_t n, out_base, tri_cursor, level;
+};
+
 struct Build8 {
     const Node* nodes;
     const Tri* tris;
@@ -142,6 +148,7 @@ struct Build8 {
     Tri* tris8;
     uint32_t max_nodes, max_tris, num_tris;
     Size8* size;
+    Level8* handed;            // what block 0 hands to the others after levels of its own
     uint32_t* sync;
     uint32_t* err;
 };
@@ -357,24 +364,39 @@ __device__ __forceinline__ void collapse_group(const Build8& B, bool have, uint3
 // (a ballot over a step's 32 slots ranks them: inner children become the next
 // level, leaf triangles are copied); a second barrier. Small levels go to as
 // few warps a block as they need, on all blocks, so their few nodes run on many
-// SMs. One launch replaces three a level and a host read-back every four: the
-// 1M-triangle soup (8 levels, 284 Ki nodes) takes 0.21 ms instead of 0.49, and a
-// rebuilt BVH with 262,144 rays against it 877 us instead of 1,131. A small level
-// costs 11 us (collapsing one node 5 us of dependent loads, two barriers 4.5, the
-// places 1.8); the 242 Ki-node level 60 to 90 us a block, issue bound (1,240 warp
-// instructions for four nodes; 1,510 before the slots were assigned in rounds and
-// the planes quantised without a search). 4 blocks an SM (59 registers) against
-// 3: 877 and 886 us; prefetching the next nodes' neighbourhoods to L1 or L2
-// changed nothing.
+// SMs. A level of at most 32 nodes, one step of a block's warps, is block 0's
+// alone: no grid barrier, until a level is larger (it then hands the state over)
+// or none is left. One launch replaces three a level and a host read-back every
+// four: the 1M-triangle soup (8 levels, 284 Ki nodes) takes 0.21 ms instead of
+// 0.49. A small level of all blocks costs 11 us (collapsing one node 5 us of
+// dependent loads, two barriers 4.5, the places 1.8), so with such levels left to
+// one block a rebuild and 1,024 rays take 103 us instead of 110 at 300 triangles,
+// 178 instead of 184 at 10,000, 568 instead of 572 at 1M. The 242 Ki-node level
+// takes 60 to 90 us a block, issue bound (1,240 warp instructions for four nodes;
+// 1,510 before the slots were assigned in rounds and the planes quantised without
+// a search). 4 blocks an SM (64 registers, 8 bytes of spills) against 3 was 877
+// against 886 us for a rebuilt 1M-triangle BVH and 262,144 rays; prefetching the
+// next nodes' neighbourhoods to L1 or L2 changed nothing.
 __global__ void __launch_bounds__(kThreads8, 4) k8_build(Build8 B) {
     __shared__ uint32_t s_rec[kWarps8][kNodesPerWarp][24];
     __shared__ int32_t s_ref[kWarps8][kNodesPerWarp][8];
     __shared__ unsigned long long s_warp[kWarps8], s_before[kWarps8], s_total[kWarps8];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t g = lane / kLanesPerNode, k = lane & (kLanesPerNode - 1);
-    const uint32_t grid = gridDim.x;
-    uint32_t n = 1, out_base = 0, tri_cursor = 0, arrived = 0, overflow = 0;
-    for (uint32_t level = 0; n != 0; ++level) {
+    uint32_t n = 1, out_base = 0, tri_cursor = 0, level = 0, arrived = 0, overflow = 0;
+    while (n != 0) {
+        const bool alone = n <= kAloneNodes;
+        if (alone && blockIdx.x != 0) {
+            grid_sync(B.sync, ++arrived * gridDim.x, B.err);
+            const uint4 h = __ldcg(reinterpret_cast<const uint4*>(B.handed));
+            n = h.x;
+            out_base = h.y;
+            tri_cursor = h.z;
+            level = h.w;
+            if (n > B.max_nodes || out_base > B.max_nodes - n) n = 0;  // only after a barrier that gave up
+            continue;
+        }
+        const uint32_t grid = alone ? 1u : gridDim.x;  // blocks that share the level
         const uint32_t* frontier = (level & 1) ? B.frontier[1] : B.frontier[0];
         const uint64_t per_block = (uint64_t)grid * kNodesPerWarp;
         const uint32_t active = (uint32_t)min((uint64_t)kWarps8, (n + per_block - 1) / per_block);  // warps a block
@@ -397,39 +419,43 @@ __global__ void __launch_bounds__(kThreads8, 4) k8_build(Build8 B) {
         }
         if (lane == 0) s_warp[warp] = (unsigned long long)inner | ((unsigned long long)leaves << 32);
         __syncthreads();
-        if (threadIdx.x == 0) {
-            unsigned long long sum = 0;
-            for (int w = 0; w < kWarps8; ++w) sum += s_warp[w];
-            B.bsum[blockIdx.x] = sum;
-        }
-        grid_sync(B.sync, ++arrived * grid, B.err);
         unsigned long long before = 0, total = 0;
-        for (uint32_t j = threadIdx.x; j < grid; j += kThreads8) {
-            const unsigned long long v = __ldcg(B.bsum + j);
-            total += v;
-            if (j < blockIdx.x) before += v;
-        }
+        if (!alone) {
+            if (threadIdx.x == 0) {
+                unsigned long long sum = 0;
+                for (int w = 0; w < kWarps8; ++w) sum += s_warp[w];
+                B.bsum[blockIdx.x] = sum;
+            }
+            grid_sync(B.sync, ++arrived * grid, B.err);
+            for (uint32_t j = threadIdx.x; j < grid; j += kThreads8) {
+                const unsigned long long v = __ldcg(B.bsum + j);
+                total += v;
+                if (j < blockIdx.x) before += v;
+            }
 #pragma unroll
-        for (int d = 16; d > 0; d >>= 1) {
-            before += __shfl_xor_sync(0xFFFFFFFFu, before, d);
-            total += __shfl_xor_sync(0xFFFFFFFFu, total, d);
+            for (int d = 16; d > 0; d >>= 1) {
+                before += __shfl_xor_sync(0xFFFFFFFFu, before, d);
+                total += __shfl_xor_sync(0xFFFFFFFFu, total, d);
+            }
+            if (lane == 0) {
+                s_before[warp] = before;
+                s_total[warp] = total;
+            }
+            __syncthreads();
+            before = 0;
+            total = 0;
         }
-        if (lane == 0) {
-            s_before[warp] = before;
-            s_total[warp] = total;
-        }
-        __syncthreads();
-        before = 0;
-        total = 0;
         for (int w = 0; w < kWarps8; ++w) {
-            before += s_before[w];
-            total += s_total[w];
+            before += alone ? 0ull : s_before[w];
+            total += alone ? s_warp[w] : s_total[w];
             if (w < warp) before += s_warp[w];
         }
         const uint32_t next_base = out_base + n;
         const uint64_t next_n = (uint32_t)total, next_tri = tri_cursor + (total >> 32);
         if (next_base + next_n > B.max_nodes || next_tri > B.max_tris || level >= kMaxLevels8) {
-            overflow = 1;  // the same for every block
+            overflow = 1;  // the same for every block that shares the level
+            if (alone && threadIdx.x == 0) *B.handed = Level8{0u, out_base, tri_cursor, level};
+            if (alone) grid_sync(B.sync, ++arrived * gridDim.x, B.err);
             break;
         }
         uint32_t in_run = (uint32_t)before, leaf_run = (uint32_t)(before >> 32);
@@ -458,10 +484,16 @@ __global__ void __launch_bounds__(kThreads8, 4) k8_build(Build8 B) {
             in_run += __popc(mi);
             leaf_run += __popc(ml);
         }
-        grid_sync(B.sync, ++arrived * grid, B.err);
         out_base = next_base;
         tri_cursor = (uint32_t)next_tri;
         n = (uint32_t)next_n;
+        ++level;
+        if (alone && n <= kAloneNodes && n != 0) {
+            __syncthreads();
+        } else {
+            if (alone && threadIdx.x == 0) *B.handed = Level8{n, out_base, tri_cursor, level};
+            grid_sync(B.sync, ++arrived * gridDim.x, B.err);
+        }
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) *B.size = Size8{out_base, tri_cursor, overflow, 0u};
 }
@@ -492,7 +524,7 @@ cudaError_t bvh8_build(BvhBuffers& b, uint32_t n, DevBuf& scratch, int num_sms, 
     const size_t o_f1 = off; off += align256(4 * maxnodes);
     const size_t o_sl = off; off += align256(32 * maxnodes);
     const size_t o_bs = off; off += align256(8 * (size_t)grid);
-    const size_t o_sz = off; off += 256;  // Size8, then the barrier counter at 64
+    const size_t o_sz = off; off += 256;  // Size8, then the barrier counter at 64 and Level8 at 128
     const size_t o_nd = off; off += align256(sizeof(Node8Q) * maxnodes);
     if ((e = scratch.ensure(off)) != cudaSuccess) return e;
     if ((e = b.tris8.ensure(sizeof(Tri) * maxtris)) != cudaSuccess) return e;
@@ -514,6 +546,7 @@ cudaError_t bvh8_build(BvhBuffers& b, uint32_t n, DevBuf& scratch, int num_sms, 
     B.num_tris = n;
     B.size = (Size8*)(base + o_sz);
     B.sync = (uint32_t*)(base + o_sz + 64);
+    B.handed = (Level8*)(base + o_sz + 128);
     B.err = &((BvhMeta*)b.meta.p)->err;
     if ((e = cudaMemsetAsync(base + o_sz, 0, 256, s)) != cudaSuccess) return e;
     for (;;) {

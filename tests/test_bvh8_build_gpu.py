@@ -45,3 +45,18 @@ def test_planes_on_steps_and_extreme_coordinates(ctx, oracle, name):
     f = np.ascontiguousarray(v, np.float32)
     _check(b, oracle, f)
     b.close()
+
+
+@pytest.mark.parametrize("outer,inner", [(120, 3000), (200, 3000), (300, 9000)])
+def test_levels_that_narrow_and_widen(ctx, oracle, outer, inner):
+    """A loose soup, a chain towards a corner and a dense cluster in it: levels such as 1, 8, 56, 1, 8, 48, 316, 597, 6
+    nodes, so the build passes from one block to all of them and back more than once."""
+    chain = sc.triangle_soup(8, seed_salt=73).reshape(8, 9) * np.float32(2.0 ** -11)
+    chain = chain + np.float32(2.0) ** -np.arange(1, 9, dtype=np.float32)[:, None]
+    dense = sc.triangle_soup(inner, seed_salt=72) * np.float32(2.0 ** -9)
+    v = np.concatenate([sc.triangle_soup(outer, seed_salt=71), chain, dense])
+    b = gr.BVH(ctx)
+    b.set_layout(gr.LAYOUT_BVH8_Q8)
+    _check(b, oracle, np.ascontiguousarray(v, np.float32))
+    _check(b, oracle, np.ascontiguousarray(v[::-1], np.float32))
+    b.close()
