@@ -789,6 +789,14 @@ __global__ void __launch_bounds__(kShadeThreads) k_mean_rgb(const double* __rest
 // Waves of up to this many paths overlap the launches of their kernels (launch.cuh).
 constexpr uint32_t kOverlapPaths = 1u << 16;
 
+// Waves of up to this many paths shade in queue order whatever their materials: a
+// launch of k_bin costs more per bounce than the divergence of the few warps that
+// a scheduler gets (14 at the line). Grouped against queue order (us, 8 bounces,
+// host image): textured 19 k paths 362 / 330, 64 Ki 441 / 414, 256 Ki 497 / 489,
+// 512 Ki 581 / 588; glossy 19 k 527 / 502, 64 Ki 692 / 668, 256 Ki 1,579 / 1,551
+// (500 k triangles), 512 Ki 1,105 / 1,142 (20 k triangles).
+constexpr uint32_t kQueueOrderPaths = 1u << 18;
+
 // One wave: clear counters, camera rays, depth_steps x (trace, shade)
 // (steps past the wave's max_depth return at once), resolve (which adds the ray counts up).
 template <int LAYOUT, int SSTACK>
@@ -1032,10 +1040,10 @@ cudaError_t run_wave(WavePool& pool, const JobDev* h_jobs, uint32_t njobs, uint3
     // the captured sequence runs exactly the wave's bounce steps (an empty step
     // still costs three launches)
     const uint32_t steps = max_depth;
-    // shade in material groups when the wave's scenes mix material types
+    // shade in material groups when a large wave's scenes mix material types
     uint32_t types = 0;
     for (uint32_t j = 0; j < njobs; ++j) types |= h_jobs[j].sc.mat_types;
-    const bool bin = __builtin_popcount(types) >= 2;
+    const bool bin = __builtin_popcount(types) >= 2 && total_paths > kQueueOrderPaths;
     const bool small = total_paths <= kOverlapPaths;
     if (!use_graph) return issue_wave(ps, max_depth, tgrid, sgrid, bin, small, s, tune);
     uint64_t key = 0x51ED270B27A3C1F5ull;

@@ -39,3 +39,27 @@ def test_short_queues_match_oracle_alone_and_packed(ctx, oracle, layout, w, h, s
         np.testing.assert_array_equal(s.accumulation()[0], want)
         s.close()
     assert st.closest_rays == sum(a[1] for a in alone) and st.shadow_rays == sum(a[2] for a in alone)
+
+
+@pytest.mark.parametrize("layout", [gr.LAYOUT_BVH2, gr.LAYOUT_BVH8_Q8])
+@pytest.mark.parametrize("w,h,spp", [(512, 256, 2), (511, 257, 2), (512, 257, 2)])
+def test_material_groups_and_queue_order_render_the_same(ctx, layout, w, h, spp):
+    """Waves of 2^18 paths and a few more (shaded in queue order up to there, in material groups above), against the same render cut into small waves, and with a scene of other materials in the wave: bit for bit."""
+    desc, other = sc.glossy_scene(w, h, level=3, glass_level=2), sc.textured_scene(64, 48)
+    got = []
+    for wave_paths in (0, w * h):
+        s = gr.Scene(ctx, desc)
+        s.set_tuning(layout, 64, 12)
+        _, st = s.render(spp, max_depth=9, seed=5, wave_paths=wave_paths)
+        assert st.device_errors == 0
+        got.append((s.accumulation()[0], st.closest_rays, st.shadow_rays))
+        s.close()
+    assert got[0][1:] == got[1][1:]
+    np.testing.assert_array_equal(got[0][0], got[1][0])
+    packed = [gr.Scene(ctx, d) for d in (desc, other)]
+    for s in packed:
+        s.set_tuning(layout, 64, 12)
+    gr.render_batch(ctx, packed, [dict(spp=spp, max_depth=9, seed=5)] * 2)
+    np.testing.assert_array_equal(packed[0].accumulation()[0], got[0][0])
+    for s in packed:
+        s.close()
