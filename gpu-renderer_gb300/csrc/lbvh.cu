@@ -212,7 +212,7 @@ __global__ void __launch_bounds__(kBlock) k_morton_hist(const float* __restrict_
 }
 
 // ---- 3. radix sort ----------------------------------------------------------------
-// Four passes of one 8-bit digit each. Tiles of 4096 keys are ranked in shared
+// Four passes of one 8-bit digit each. Tiles of 512 to 4096 keys are ranked in shared
 // memory (warp multi-split by ballots, stable in input order), the tile's
 // per-digit counts are prefixed over the tiles before it, and keys are written
 // out grouped by digit. The prefix comes from a grid barrier and a scan of every
@@ -270,7 +270,10 @@ __device__ __forceinline__ uint32_t match_digit(uint32_t d) {
 // digit counts itself (one grid barrier); more tiles scan the counts first.
 constexpr uint32_t kSumTiles = 64;
 
-constexpr size_t kOsSmem = sizeof(uint32_t) * (kOsWarps * 256 + 256 + 256 + 2 * kOsTile + 2 * kOsWarps + 1);
+constexpr size_t os_smem(int items) {
+    return sizeof(uint32_t) * (kOsWarps * 256 + 256 + 256 + 2 * (kOsThreads * items) + 2 * kOsWarps + 1);
+}
+constexpr size_t kOsSmem = os_smem(kOsItems);
 
 // One tile of one sort pass: ranks the tile's keys by the pass's digit, finds
 // where each digit's run of the tile starts in the output, and writes the
@@ -281,29 +284,30 @@ constexpr size_t kOsSmem = sizeof(uint32_t) * (kOsWarps * 256 + 256 + 256 + 2 * 
 // a grid barrier (`barrier` is its index in the launch): up to kSumTiles tiles
 // each tile sums the columns itself; beyond, the blocks scan the columns over
 // the tiles and a second grid barrier follows.
-template <bool COOP>
+template <bool COOP, int ITEMS>
 __device__ __forceinline__ void sort_tile(const uint32_t* __restrict__ kin, const uint32_t* __restrict__ vin,
                                           uint32_t* __restrict__ kout, uint32_t* __restrict__ vout, uint32_t n,
                                           int pass, const uint32_t* __restrict__ hist, uint32_t tile,
                                           uint32_t* __restrict__ status, uint32_t* sync_ctr, uint32_t barrier,
                                           uint32_t* __restrict__ err, uint32_t* smem) {
+    constexpr int kTile = kOsThreads * ITEMS;
     uint32_t* s_wcnt = smem;                       // [warps][256]
     uint32_t* s_dstart = s_wcnt + kOsWarps * 256;  // [256] tile-local digit starts
     uint32_t* s_gbase = s_dstart + 256;            // [256] global digit bases
     uint32_t* s_keys = s_gbase + 256;              // [tile]
-    uint32_t* s_vals = s_keys + kOsTile;           // [tile]
-    unsigned long long* s_warp = reinterpret_cast<unsigned long long*>(s_vals + kOsTile);  // [warps] scan scratch
+    uint32_t* s_vals = s_keys + kTile;           // [tile]
+    unsigned long long* s_warp = reinterpret_cast<unsigned long long*>(s_vals + kTile);  // [warps] scan scratch
 
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int shift = 8 * pass;
     for (int i = threadIdx.x; i < kOsWarps * 256; i += kOsThreads) s_wcnt[i] = 0;
     __syncthreads();
-    const uint64_t base = (uint64_t)tile * kOsTile;
+    const uint64_t base = (uint64_t)tile * kTile;
 
-    uint32_t key[kOsItems], val[kOsItems], rank[kOsItems], dig[kOsItems];
+    uint32_t key[ITEMS], val[ITEMS], rank[ITEMS], dig[ITEMS];
 #pragma unroll
-    for (int j = 0; j < kOsItems; ++j) {
-        const uint64_t idx = base + warp * (32 * kOsItems) + j * 32 + lane;
+    for (int j = 0; j < ITEMS; ++j) {
+        const uint64_t idx = base + warp * (32 * ITEMS) + j * 32 + lane;
         const bool ok = idx < n;
         key[j] = ok ? (COOP ? __ldcg(kin + idx) : kin[idx]) : 0u;
         val[j] = ok ? (COOP ? __ldcg(vin + idx) : vin[idx]) : 0u;
@@ -312,7 +316,7 @@ __device__ __forceinline__ void sort_tile(const uint32_t* __restrict__ kin, cons
     const uint32_t ltmask = lanemask_lt();
     uint32_t* wc = s_wcnt + warp * 256;
 #pragma unroll
-    for (int j = 0; j < kOsItems; ++j) {
+    for (int j = 0; j < ITEMS; ++j) {
         const uint32_t d = dig[j];
         const uint32_t peers = match_digit(d);
         const uint32_t lt = __popc(peers & ltmask);
@@ -338,7 +342,7 @@ __device__ __forceinline__ void sort_tile(const uint32_t* __restrict__ kin, cons
     __syncthreads();
     // one scan gives the tile-local digit starts (low word) and the pass's
     // global digit starts from the histogram (high word; the tile's counts sum
-    // to at most kOsTile, so the low word never carries)
+    // to at most kTile, so the low word never carries)
     unsigned long long tot;
     const unsigned long long both = block_exclusive_scan<kOsThreads>(
         threadIdx.x < 256 ? ((unsigned long long)hist[256 * pass + threadIdx.x] << 32) | cnt : 0ull, s_warp, &tot);
@@ -412,7 +416,7 @@ __device__ __forceinline__ void sort_tile(const uint32_t* __restrict__ kin, cons
     }
     __syncthreads();
 #pragma unroll
-    for (int j = 0; j < kOsItems; ++j) {
+    for (int j = 0; j < ITEMS; ++j) {
         const uint32_t d = dig[j];
         if (d < 256u) {
             const uint32_t r = s_dstart[d] + s_wcnt[warp * 256 + d] + rank[j];
@@ -422,7 +426,7 @@ __device__ __forceinline__ void sort_tile(const uint32_t* __restrict__ kin, cons
     }
     __syncthreads();
     const uint64_t left = (uint64_t)n - base;
-    const uint32_t valid = left < (uint64_t)kOsTile ? (uint32_t)left : (uint32_t)kOsTile;
+    const uint32_t valid = left < (uint64_t)kTile ? (uint32_t)left : (uint32_t)kTile;
     for (uint32_t i = threadIdx.x; i < valid; i += kOsThreads) {
         const uint32_t k = s_keys[i];
         const uint32_t d = (k >> shift) & 0xFFu;
@@ -448,7 +452,7 @@ __global__ void __launch_bounds__(kOsThreads, 2) k_onesweep(const uint32_t* __re
     wait_for_previous();
     if (threadIdx.x == 0) s_tile = atomicAdd(tile_ctr + pass, 1u);
     __syncthreads();
-    sort_tile<false>(kin, vin, kout, vout, n, pass, hist, s_tile, status, nullptr, 0, err, smem);
+    sort_tile<false, kOsItems>(kin, vin, kout, vout, n, pass, hist, s_tile, status, nullptr, 0, err, smem);
 }
 
 // All four sort passes in one cooperative launch, one block per tile (every
@@ -457,6 +461,7 @@ __global__ void __launch_bounds__(kOsThreads, 2) k_onesweep(const uint32_t* __re
 // after the counts are scanned (more than kSumTiles tiles), and after the
 // tiles are written (before the next pass reads them and overwrites the
 // counts).
+template <int ITEMS>
 __global__ void __launch_bounds__(kOsThreads, 2) k_sort_coop(uint32_t* key_a, uint32_t* val_a, uint32_t* key_b,
                                                           uint32_t* val_b, uint32_t n,
                                                           const uint32_t* __restrict__ hist, uint32_t* counts,
@@ -465,7 +470,7 @@ __global__ void __launch_bounds__(kOsThreads, 2) k_sort_coop(uint32_t* key_a, ui
     const uint32_t per_pass = gridDim.x <= kSumTiles ? 2 : 3;  // grid barriers a pass
     for (int pass = 0; pass < 4; ++pass) {
         const bool even = (pass & 1) == 0;
-        sort_tile<true>(even ? key_a : key_b, even ? val_a : val_b, even ? key_b : key_a, even ? val_b : val_a, n,
+        sort_tile<true, ITEMS>(even ? key_a : key_b, even ? val_a : val_b, even ? key_b : key_a, even ? val_b : val_a, n,
                         pass, hist, blockIdx.x, counts, sync_ctr, per_pass * pass, err, smem);
         if (pass < 3) grid_sync(sync_ctr, per_pass * (pass + 1) * gridDim.x, err);
     }
@@ -1071,8 +1076,12 @@ cudaError_t lookback_probe(uint32_t polls, uint32_t* h_err, cudaStream_t s) {
 
 namespace {
 
+uint32_t tiles_of(uint32_t n, int items) {
+    return (uint32_t)(((uint64_t)n + kOsThreads * items - 1) / (kOsThreads * items));
+}
+
 // How many sort tiles one cooperative launch can hold on the current device
-// (resident blocks of k_sort_coop per SM times the SMs; 0 without cooperative
+// (resident blocks of the largest k_sort_coop per SM times the SMs; 0 without cooperative
 // launch), looked up once per device.
 cudaError_t sort_coop_capacity(int num_sms, int* tiles) {
     static std::mutex mu;
@@ -1085,10 +1094,10 @@ cudaError_t sort_coop_capacity(int num_sms, int* tiles) {
     if (dev < 0 || dev >= 64 || !known[dev]) {
         int coop = 0, per_sm = 0;
         if ((e = cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev)) != cudaSuccess) return e;
-        if ((e = cudaFuncSetAttribute(k_sort_coop, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kOsSmem)) !=
+        if ((e = cudaFuncSetAttribute(k_sort_coop<kOsItems>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kOsSmem)) !=
             cudaSuccess)
             return e;
-        if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_sort_coop, kOsThreads, kOsSmem)) !=
+        if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_sort_coop<kOsItems>, kOsThreads, kOsSmem)) !=
             cudaSuccess)
             return e;
         const int cap = coop ? per_sm * num_sms : 0;
@@ -1101,6 +1110,36 @@ cudaError_t sort_coop_capacity(int num_sms, int* tiles) {
     }
     *tiles = cached[dev];
     return cudaSuccess;
+}
+
+// Keys a thread of the cooperative sort ranks (tiles of 512 times that). A pass
+// lasts as long as its busiest SM, and ranking is most of it, so tiles are as small
+// as a limit on their number allows: one tile, which has no barriers, up to 3,072
+// keys (3,001 triangles built in 37.8 us, in several tiles 39.8; 4,000 in 41.9 and
+// 39.9); else kSumTiles, beyond which the counts take a scan and a barrier more a
+// pass (98,304 triangles: 64 tiles 70.7, 96 tiles 77.9); else one tile an SM; else
+// what is resident. Builds with this rule against 8 keys a thread always (us):
+// 600 triangles 37 / 29, 5,000 47 / 39, 30,000 61 / 49, 100,003 80 / 71, 131,072
+// 86 / 79, 200,000 95 / 91, 300,000 119 / 108, 800,000 166 / 159, 1 M 183.5 / 179.
+int sort_items(uint32_t n, int num_sms, int resident) {
+    const uint32_t limits[] = {n <= 6 * kOsThreads ? 1u : kSumTiles, (uint32_t)num_sms, (uint32_t)resident};
+    for (uint32_t limit : limits)
+        for (int items = n <= kOsThreads ? 1 : 2; items <= kOsItems; ++items)
+            if (tiles_of(n, items) <= std::min(limit, (uint32_t)resident)) return items;
+    return kOsItems;
+}
+
+const void* sort_coop_kernel(int items) {
+    switch (items) {
+        case 1: return (const void*)k_sort_coop<1>;
+        case 2: return (const void*)k_sort_coop<2>;
+        case 3: return (const void*)k_sort_coop<3>;
+        case 4: return (const void*)k_sort_coop<4>;
+        case 5: return (const void*)k_sort_coop<5>;
+        case 6: return (const void*)k_sort_coop<6>;
+        case 7: return (const void*)k_sort_coop<7>;
+        default: return (const void*)k_sort_coop<kOsItems>;
+    }
 }
 
 // Builds of up to this many triangles overlap the launches of their kernels (launch.cuh).
@@ -1140,7 +1179,14 @@ cudaError_t launch_build(const float* d_verts, uint32_t n, const Scratch& s, Nod
         uint32_t* sync_ctr = s.tile_ctr + 8;
         void* args[] = {&code, &prim, (void*)&s.keys_alt, (void*)&s.vals_alt, &n, (void*)&s.hist,
                         (void*)&s.os_status, &sync_ctr, &err};
-        e = cudaLaunchCooperativeKernel((const void*)k_sort_coop, dim3(os_tiles), dim3(kOsThreads), args, kOsSmem, st);
+        int items = sort_items(n, num_sms, coop_tiles);
+        for (;;) {
+            e = cudaLaunchCooperativeKernel(sort_coop_kernel(items), dim3(tiles_of(n, items)), dim3(kOsThreads), args,
+                                            os_smem(items), st);
+            if (e != cudaErrorCooperativeLaunchTooLarge || items == kOsItems) break;
+            (void)cudaGetLastError();
+            items = kOsItems;  // fewer, larger tiles
+        }
         if (e == cudaSuccess) {
             sorted = true;
         } else if (e == cudaErrorCooperativeLaunchTooLarge) {
