@@ -622,7 +622,7 @@ __device__ __forceinline__ bool trace_step(L_& L, int2* s_stack, int2* l_stack, 
 }
 
 // A warp refills its idle lanes once at least REFILL of them are idle. The
-// ray-query kernels use 4 (a ray loads in two 16-byte reads; 2, 6 and 8
+// ray-query kernels use 4 (a ray loads in two 16-byte reads; 6 is the same, 2 and 8
 // measured slower), with binary nodes 8 (below); the render's queue kernels use 12
 // (a queued ray also looks up its job and scene; glossy 1024 x 768 x 64 spp: 72.4 ms
 // at 8 and 12, 74.5 at 4, 74.1 at 16).
