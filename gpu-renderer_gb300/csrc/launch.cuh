@@ -4,6 +4,15 @@
 // writes are visible. Every kernel launched so calls it before it touches global
 // memory, on every path, so the chain of kernels keeps the stream's order.
 //
+// Such a grid exists while the kernel before it still writes, so what that kernel
+// writes is not read-only for the grid's lifetime, as __ldg and const __restrict__
+// parameters promise, and __restrict__ tells the compiler that the wait does not touch
+// the memory: such loads and stores may be moved above the wait. So these kernels take
+// plain pointers, which the wait orders. Data written before the kernel before may be
+// read either way: that kernel has waited for its writer before it lets this one
+// start. The first kernel of a chain follows whatever the caller launched, so it reads
+// the caller's data through plain pointers too.
+//
 // It pays where kernels take microseconds and the 1-2 us between two of them count:
 // LBVH of 100,003 triangles 86.3 -> 79.7 us, of 3,001 with a trace of 2,048 rays
 // 108 -> 98 us, a 160 x 120 x 1 spp preview 422 -> 414 us. Where a kernel's last blocks

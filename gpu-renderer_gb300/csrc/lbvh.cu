@@ -38,11 +38,13 @@ struct Box3 {
     float lo[3], hi[3];
 };
 
-__device__ __forceinline__ Box3 tri_box(const float* __restrict__ v, uint64_t i) {
+// READ_ONLY: nothing writes the vertices while this kernel's grid exists (launch.cuh).
+template <bool READ_ONLY>
+__device__ __forceinline__ Box3 tri_box(const float* v, uint64_t i) {
     const float* p = v + 9ull * i;
     float a[9];
 #pragma unroll
-    for (int k = 0; k < 9; ++k) a[k] = __ldg(p + k);
+    for (int k = 0; k < 9; ++k) a[k] = READ_ONLY ? __ldg(p + k) : p[k];
     Box3 b;
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
@@ -125,10 +127,12 @@ __device__ __forceinline__ float block_bounds(float lo[3], float hi[3]) {
 // kernel, it also clears what must start at zero: the header's other words, the
 // digit histograms and the sort's counters (`zero`, `nzero` words). Two memsets
 // and a copy of the error word, 2 us each, did that before: 100,003 triangles
-// 92.6 -> 86.2 us, 3,001 with a trace of 2,048 rays 117.6 -> 111.6 us.
-__global__ void __launch_bounds__(kBlock) k_centroid(const float* __restrict__ verts, uint32_t n,
-                                                     float* __restrict__ partial, uint32_t* __restrict__ done,
-                                                     uint32_t* __restrict__ zero, uint32_t nzero, BvhMeta* meta) {
+// 92.6 -> 86.2 us, 3,001 with a trace of 2,048 rays 117.6 -> 111.6 us. The vertices
+// may come from the kernel before it, so it reads them coherently; the build's later
+// kernels start when that one has ended.
+__global__ void __launch_bounds__(kBlock) k_centroid(const float* verts, uint32_t n,
+                                                     float* partial, uint32_t* done, uint32_t* zero, uint32_t nzero,
+                                                     BvhMeta* meta) {
     wait_for_previous();
     if (blockIdx.x == 0) {
         for (uint32_t i = threadIdx.x; i < nzero; i += kBlock) zero[i] = 0;
@@ -139,7 +143,7 @@ __global__ void __launch_bounds__(kBlock) k_centroid(const float* __restrict__ v
     }
     float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
     for (uint32_t i = blockIdx.x * kBlock + threadIdx.x; i < n; i += gridDim.x * kBlock) {
-        Box3 b = tri_box(verts, i);
+        Box3 b = tri_box<false>(verts, i);
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
             float c = __fmul_rn(__fadd_rn(b.lo[k], b.hi[k]), 0.5f);  // AABB::centroid
@@ -177,9 +181,8 @@ __global__ void __launch_bounds__(kBlock) k_centroid(const float* __restrict__ v
 // Also clears the sort's status words (`status`, `nstatus` words), which the
 // look-back passes need at zero.
 __global__ void __launch_bounds__(kBlock) k_morton_hist(const float* __restrict__ verts, uint32_t n,
-                                                        const BvhMeta* __restrict__ meta, uint32_t* __restrict__ keys,
-                                                        uint32_t* __restrict__ vals, uint32_t* __restrict__ hist,
-                                                        uint32_t* __restrict__ status, uint32_t nstatus) {
+                                                        const BvhMeta* meta, uint32_t* keys, uint32_t* vals,
+                                                        uint32_t* hist, uint32_t* status, uint32_t nstatus) {
     __shared__ uint32_t s_hist[4 * 256];
     for (int i = threadIdx.x; i < 4 * 256; i += kBlock) s_hist[i] = 0;
     wait_for_previous();
@@ -189,7 +192,7 @@ __global__ void __launch_bounds__(kBlock) k_morton_hist(const float* __restrict_
 #pragma unroll
     for (int k = 0; k < 3; ++k) { blo[k] = meta->cbox[k]; bhi[k] = meta->cbox[3 + k]; }
     for (uint32_t i = blockIdx.x * kBlock + threadIdx.x; i < n; i += gridDim.x * kBlock) {
-        Box3 b = tri_box(verts, i);
+        Box3 b = tri_box<true>(verts, i);
         uint32_t cell[3];
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
@@ -285,9 +288,8 @@ constexpr size_t kOsSmem = os_smem(kOsItems);
 // each tile sums the columns itself; beyond, the blocks scan the columns over
 // the tiles and a second grid barrier follows.
 template <bool COOP, int ITEMS>
-__device__ __forceinline__ void sort_tile(const uint32_t* __restrict__ kin, const uint32_t* __restrict__ vin,
-                                          uint32_t* __restrict__ kout, uint32_t* __restrict__ vout, uint32_t n,
-                                          int pass, const uint32_t* __restrict__ hist, uint32_t tile,
+__device__ __forceinline__ void sort_tile(const uint32_t* kin, const uint32_t* vin, uint32_t* __restrict__ kout,
+                                          uint32_t* __restrict__ vout, uint32_t n, int pass, const uint32_t* hist, uint32_t tile,
                                           uint32_t* __restrict__ status, uint32_t* sync_ctr, uint32_t barrier,
                                           uint32_t* __restrict__ err, uint32_t* smem) {
     constexpr int kTile = kOsThreads * ITEMS;
@@ -442,11 +444,9 @@ __device__ __forceinline__ void sort_tile(const uint32_t* __restrict__ kin, cons
 
 // One sort pass, tiles taken in launch order from `tile_ctr` (so a tile's
 // predecessors have started: the look-back's waits end).
-__global__ void __launch_bounds__(kOsThreads, 2) k_onesweep(const uint32_t* __restrict__ kin, const uint32_t* __restrict__ vin,
-                                                         uint32_t* __restrict__ kout, uint32_t* __restrict__ vout,
-                                                         uint32_t n, int pass, const uint32_t* __restrict__ hist,
-                                                         uint32_t* __restrict__ status, uint32_t* __restrict__ tile_ctr,
-                                                         uint32_t* __restrict__ err) {
+__global__ void __launch_bounds__(kOsThreads, 2) k_onesweep(const uint32_t* kin, const uint32_t* vin, uint32_t* kout,
+                                                         uint32_t* vout, uint32_t n, int pass, const uint32_t* hist,
+                                                         uint32_t* status, uint32_t* tile_ctr, uint32_t* err) {
     extern __shared__ uint32_t smem[];
     __shared__ uint32_t s_tile;
     wait_for_previous();
@@ -496,7 +496,7 @@ __global__ void __launch_bounds__(kOsThreads, 2) k_sort_coop(uint32_t* key_a, ui
 // Depth of gap g (codes g and g + 1 equal) in the midpoint subtree of its run:
 // the run's ends by exponential then binary search over the sorted codes, then
 // a descent from the run's root split.
-__device__ __forceinline__ uint32_t run_depth(const uint32_t* __restrict__ code, uint32_t n, uint32_t g,
+__device__ __forceinline__ uint32_t run_depth(const uint32_t* code, uint32_t n, uint32_t g,
                                               uint32_t* __restrict__ err) {
     const uint32_t c = code[g];
     int64_t good = g, bad = -1;  // code[good] == c; code[bad] < c (or bad = -1)
@@ -535,9 +535,8 @@ __device__ __forceinline__ uint32_t run_depth(const uint32_t* __restrict__ code,
     return depth;
 }
 
-__global__ void __launch_bounds__(kBlock) k_gaps(const uint32_t* __restrict__ code, uint32_t n,
-                                                 uint8_t* __restrict__ level, uint32_t* __restrict__ done,
-                                                 uint32_t* __restrict__ err) {
+__global__ void __launch_bounds__(kBlock) k_gaps(const uint32_t* code, uint32_t n,
+                                                 uint8_t* level, uint32_t* done, uint32_t* err) {
     wait_for_previous();
     // zero already, unless builds sharing the scratch overlapped: a build leaves it so for the next
     if (blockIdx.x == 0 && threadIdx.x == 0) *done = 0;
@@ -705,9 +704,8 @@ __device__ __forceinline__ uint32_t atomic_or_acq_rel_cta(uint32_t* p, uint32_t 
 // leaf parent and its gap's node: the whole record if both children arrived,
 // else the one child's slot and far word, and the gap's arrival bit, for part 2.
 __global__ void __launch_bounds__(kRefitChunk) k_climb_chunk(const float* __restrict__ verts, uint32_t n,
-                                                             const uint32_t* __restrict__ prim,
-                                                             const uint8_t* __restrict__ level, ClimbOut o,
-                                                             Tri* __restrict__ tris) {
+                                                             const uint32_t* prim, const uint8_t* level, ClimbOut o,
+                                                             Tri* tris) {
     __shared__ uint32_t s_mask[kRefitChunk];
     __shared__ uint32_t s_parent[kRefitChunk];
     __shared__ __align__(16) float s_box[kRefitChunk][2][6];  // per gap and slot: lo.xyz, hi.xyz
@@ -736,8 +734,8 @@ __global__ void __launch_bounds__(kRefitChunk) k_climb_chunk(const float* __rest
             Sub s;
             s.me = ~(int32_t)p;
             s.lo = s.hi = p;
-            s.llo = p > 0 ? (int32_t)__ldg(level + p - 1) : -1;
-            s.lhi = p + 1 < n ? (int32_t)__ldg(level + p) : -1;
+            s.llo = p > 0 ? (int32_t)level[p - 1] : -1;
+            s.lhi = p + 1 < n ? (int32_t)level[p] : -1;
 #pragma unroll
             for (int k = 0; k < 3; ++k) {
                 s.box.lo[k] = fminf(fminf(a[k], a[3 + k]), a[6 + k]);

@@ -393,10 +393,10 @@ __device__ __forceinline__ uint32_t job_bvh(const JobDev* jobs, uint32_t j, cons
 template <int LAYOUT>
 struct WaveSrc {
     using Index = uint32_t;
-    const float4* __restrict__ rays;
-    const float4* __restrict__ srays;
-    const float4* __restrict__ con;
-    float4* __restrict__ hits;
+    const float4* rays;  // this and the next two: written by the kernel before this one (launch.cuh)
+    const float4* srays;
+    const float4* con;
+    float4* hits;
     float4* acc;
     const JobDev* jobs;
     uint32_t nclosest, n;  // path state for 2^32 rays does not fit the GPU's memory, with room for the counter
@@ -405,8 +405,8 @@ struct WaveSrc {
     __device__ __forceinline__ uint32_t load(uint32_t i, float4& r0, float4& r1, const void*& nd, const Tri*& tr) const {
         const bool sh = any(i);
         const float4* r = sh ? srays + 2ull * (i - nclosest) : rays + 2ull * i;
-        r0 = __ldg(r);
-        r1 = __ldg(r + 1);
+        r0 = r[0];
+        r1 = r[1];
         const uint32_t root = job_bvh<LAYOUT>(jobs, __float_as_uint(r1.w), nd, tr);
         r1.z = sh ? kShadowTmin : tmin;
         r1.w = sh ? kShadowTmax : tmax;
@@ -420,7 +420,7 @@ struct WaveSrc {
             return;
         }
         if (l.best_prim != 0xFFFFFFFFu) return;
-        const float4 c = __ldg(con + (i - nclosest));
+        const float4 c = con[i - nclosest];
         const uint32_t pid = __float_as_uint(c.w);
         float4 a = acc[pid];
         a.x += c.x;
@@ -729,7 +729,7 @@ __global__ void __launch_bounds__(kShadeThreads) k_resolve(Paths ps) {
             float4 a[8];
 #pragma unroll
             for (int k = 0; k < 8; ++k)
-                if (s0 + k < samples) a[k] = __ldg(acc + (size_t)(s0 + k) * npix);
+                if (s0 + k < samples) a[k] = acc[(size_t)(s0 + k) * npix];
 #pragma unroll
             for (int k = 0; k < 8; ++k) {
                 if (s0 + k >= samples) break;
