@@ -124,10 +124,12 @@ __device__ __forceinline__ float half_area(const CBox& b) {
     return __fadd_rn(__fadd_rn(__fmul_rn(dx, dy), __fmul_rn(dy, dz)), __fmul_rn(dz, dx));
 }
 
-// What the host reads back: nodes and leaf triangles written, and whether a
-// capacity was exceeded (the build then stopped with no more writes).
+// What the host reads back: nodes and leaf triangles written, whether a
+// capacity was exceeded (the build then stopped with no more writes), and the
+// error bits with which the nodes cannot be traversed: a barrier gave up, here or
+// in the binary build, or a reference was out of range (`failed` starts at zero).
 struct Size8 {
-    uint32_t nodes, tris, overflow, pad;
+    uint32_t nodes, tris, overflow, failed;
 };
 
 // Where the build stands between two levels.
@@ -152,6 +154,12 @@ struct Build8 {
     uint32_t* sync;
     uint32_t* err;
 };
+
+// A reference that cannot be in a sound binary tree was seen and skipped.
+__device__ __noinline__ void out_of_range(const Build8& B) {
+    atomicOr(B.err, ERR_RANGE);
+    atomicOr(&B.size->failed, (uint32_t)ERR_RANGE);
+}
 
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
@@ -287,7 +295,7 @@ __device__ __forceinline__ void collapse_group(const Build8& B, bool have, uint3
                 if (rows >> s & 1u) col[s] = -INFINITY;
             }
         }
-        if (left != 0 && k == 0) atomicOr(B.err, ERR_RANGE);  // cannot happen
+        if (left != 0 && k == 0) out_of_range(B);  // cannot happen
     } else {
         // an infinite or NaN score in the warp: fold the group's pairs in order, as one thread would
         for (int it = 0; it < 8; ++it) {
@@ -384,16 +392,19 @@ __global__ void __launch_bounds__(kThreads8, 4) k8_build(Build8 B) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t g = lane / kLanesPerNode, k = lane & (kLanesPerNode - 1);
     uint32_t n = 1, out_base = 0, tri_cursor = 0, level = 0, arrived = 0, overflow = 0;
+    // A block whose barrier gave up leaves; it does not arrive again, so the others'
+    // next barrier gives up too.
+    bool met = true;
     while (n != 0) {
         const bool alone = n <= kAloneNodes;
         if (alone && blockIdx.x != 0) {
-            grid_sync(B.sync, ++arrived * gridDim.x, B.err);
+            met = grid_sync(B.sync, ++arrived * gridDim.x, B.err);
+            if (!met) break;
             const uint4 h = __ldcg(reinterpret_cast<const uint4*>(B.handed));
             n = h.x;
             out_base = h.y;
             tri_cursor = h.z;
             level = h.w;
-            if (n > B.max_nodes || out_base > B.max_nodes - n) n = 0;  // only after a barrier that gave up
             continue;
         }
         const uint32_t grid = alone ? 1u : gridDim.x;  // blocks that share the level
@@ -410,7 +421,7 @@ __global__ void __launch_bounds__(kThreads8, 4) k8_build(Build8 B) {
             bool have = i < end;
             const uint32_t id = !have ? 0u : (level == 0 ? B.meta->root : __ldcg(frontier + i));
             if (have && id >= B.max_nodes) {
-                atomicOr(B.err, ERR_RANGE);
+                out_of_range(B);
                 have = false;
             }
             const uint32_t at = out_base + i;
@@ -426,7 +437,8 @@ __global__ void __launch_bounds__(kThreads8, 4) k8_build(Build8 B) {
                 for (int w = 0; w < kWarps8; ++w) sum += s_warp[w];
                 B.bsum[blockIdx.x] = sum;
             }
-            grid_sync(B.sync, ++arrived * grid, B.err);
+            met = grid_sync(B.sync, ++arrived * grid, B.err);
+            if (!met) break;
             for (uint32_t j = threadIdx.x; j < grid; j += kThreads8) {
                 const unsigned long long v = __ldcg(B.bsum + j);
                 total += v;
@@ -455,7 +467,7 @@ __global__ void __launch_bounds__(kThreads8, 4) k8_build(Build8 B) {
         if (next_base + next_n > B.max_nodes || next_tri > B.max_tris || level >= kMaxLevels8) {
             overflow = 1;  // the same for every block that shares the level
             if (alone && threadIdx.x == 0) *B.handed = Level8{0u, out_base, tri_cursor, level};
-            if (alone) grid_sync(B.sync, ++arrived * gridDim.x, B.err);
+            if (alone) met = grid_sync(B.sync, ++arrived * gridDim.x, B.err);
             break;
         }
         uint32_t in_run = (uint32_t)before, leaf_run = (uint32_t)(before >> 32);
@@ -479,7 +491,7 @@ __global__ void __launch_bounds__(kThreads8, 4) k8_build(Build8 B) {
             } else if (r != kEmptySlot) {
                 const uint32_t to = tri_cursor + leaf_run + __popc(ml & lt), from = (uint32_t)(~r);
                 if (to < B.max_tris && from < B.num_tris) B.tris8[to] = B.tris[from];
-                else atomicOr(B.err, ERR_RANGE);
+                else out_of_range(B);
             }
             in_run += __popc(mi);
             leaf_run += __popc(ml);
@@ -492,10 +504,19 @@ __global__ void __launch_bounds__(kThreads8, 4) k8_build(Build8 B) {
             __syncthreads();
         } else {
             if (alone && threadIdx.x == 0) *B.handed = Level8{n, out_base, tri_cursor, level};
-            grid_sync(B.sync, ++arrived * gridDim.x, B.err);
+            met = grid_sync(B.sync, ++arrived * gridDim.x, B.err);
+            if (!met) break;
         }
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) *B.size = Size8{out_base, tri_cursor, overflow, 0u};
+    if (threadIdx.x != 0) return;
+    uint32_t failed = met ? 0u : (uint32_t)ERR_TIMEOUT;
+    if (blockIdx.x == 0) {
+        B.size->nodes = out_base;
+        B.size->tris = tri_cursor;
+        B.size->overflow = overflow;
+        failed |= __ldcg(B.err) & ERR_TIMEOUT;  // the binary nodes are incomplete
+    }
+    if (failed) atomicOr(&B.size->failed, failed);
 }
 
 size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
@@ -565,7 +586,8 @@ cudaError_t bvh8_build(BvhBuffers& b, uint32_t n, DevBuf& scratch, int num_sms, 
     Size8 h{};
     if ((e = cudaMemcpyAsync(&h, B.size, sizeof(h), cudaMemcpyDeviceToHost, s)) != cudaSuccess) return e;
     if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return e;
-    if (h.overflow) return cudaErrorInvalidValue;
+    if (h.failed & ERR_TIMEOUT) return cudaErrorLaunchTimeout;
+    if (h.overflow || h.failed) return cudaErrorInvalidValue;
     if (h.nodes > B.cap) {  // the layout's array grows: what it held stays in place
         DevBuf grown;
         if ((e = grown.ensure(sizeof(Node8Q) * h.nodes)) != cudaSuccess) return e;

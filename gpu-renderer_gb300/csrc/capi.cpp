@@ -94,6 +94,7 @@ gr_status cuda_fail(gr_ctx* ctx, cudaError_t e, const char* where) {
     if (ctx) {
         ctx->last_error = std::string(where) + ": " + cudaGetErrorString(e);
     }
+    if (e == cudaErrorLaunchTimeout) return fail(ctx, GR_ERR_TIMEOUT, "device wait timed out");  // bvh8_build's
     return e == cudaErrorMemoryAllocation ? GR_ERR_OOM_BUDGET : GR_ERR_CUDA;
 }
 
@@ -120,6 +121,15 @@ gr::BvhDevice device_view(gr_bvh* bvh) {
     v.meta = (const gr::BvhMeta*)bvh->buf.meta.p;
     v.n = bvh->n;
     return v;
+}
+
+bool layout_built(const gr_bvh* bvh, int layout) {
+    switch (layout) {
+        case gr::kLayoutBvh4: return bvh->built4;
+        case gr::kLayoutBvh4Q8: return bvh->built4q;
+        case gr::kLayoutBvh8Q8: return bvh->built8;
+        default: return bvh->built;
+    }
 }
 
 // Builds the derived node layout `layout` if it is not current (binary nodes
@@ -317,6 +327,8 @@ namespace {
 gr_status trace_on(gr_bvh* bvh, const gr_ray* d_rays, uint64_t n, gr_hit* d_hits, int any_hit, cudaStream_t s,
                    size_t counter_offset) {
     gr_ctx* ctx = bvh->ctx;
+    if (!layout_built(bvh, bvh->layout))  // gr_bvh_build failed after the binary nodes
+        return fail(ctx, GR_ERR_INVALID, "gr_trace: the layout's nodes are not built");
     unsigned long long* counter = (unsigned long long*)((char*)ctx->counter.p + counter_offset);
     uint32_t* err = (uint32_t*)((char*)ctx->counter.p + 64);
     gr::TraceTuning tune;
@@ -433,6 +445,14 @@ extern "C" gr_status gr_diag_bounded_wait(gr_ctx* ctx, uint32_t polls, uint32_t*
     GR_CUDA(ctx, gr::lookback_probe(polls, &bits, ctx->stream));
     if (err_bits) *err_bits = bits;
     if (bits & gr::ERR_TIMEOUT) return fail(ctx, GR_ERR_TIMEOUT, "gr_diag_bounded_wait: the wait gave up");
+    return GR_OK;
+}
+
+extern "C" gr_status gr_diag_set_build_error(gr_bvh* bvh, uint32_t bits) {
+    if (!bvh || !bvh->built) return GR_ERR_INVALID;
+    GR_CUDA(bvh->ctx, cudaSetDevice(bvh->ctx->device));
+    GR_CUDA(bvh->ctx, cudaDeviceSynchronize());
+    GR_CUDA(bvh->ctx, cudaMemcpy(&((gr::BvhMeta*)bvh->buf.meta.p)->err, &bits, 4, cudaMemcpyHostToDevice));
     return GR_OK;
 }
 

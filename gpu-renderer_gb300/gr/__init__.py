@@ -73,6 +73,7 @@ def load():
         "gr_scene_get_tuning": ([_P, _P, ctypes.POINTER(ctypes.c_uint32)], ctypes.c_int),
         "gr_scene_layout": ([_P], ctypes.c_int),
         "gr_diag_bounded_wait": ([_P, ctypes.c_uint32, ctypes.POINTER(ctypes.c_uint32)], ctypes.c_int),
+        "gr_diag_set_build_error": ([_P, ctypes.c_uint32], ctypes.c_int),
     }
     for name, (args, res) in sig.items():
         fn = getattr(L, name)

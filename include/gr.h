@@ -383,6 +383,10 @@ gr_status gr_scene_rgba8_host(gr_scene* scene, uint32_t* h_rgba);
  * out, so it returns GR_ERR_TIMEOUT with the device error bits (ERR_TIMEOUT = 1)
  * in *err_bits. */
 gr_status gr_diag_bounded_wait(gr_ctx* ctx, uint32_t polls, uint32_t* err_bits);
+/* Sets the error word that a BVH's build left in its header, as a build whose
+ * device wait gave up would (1): what is derived from the BVH then reports it.
+ * Waits for the device. */
+gr_status gr_diag_set_build_error(gr_bvh* bvh, uint32_t bits);
 
 /* ---- image files: FrameBuffer::output / WriteImage (framebuffer.cpp:11-26, imageio.cpp:59-82) ----
  * Writes a linear RGB image (width x height x 3 floats, row 0 = the first
