@@ -393,9 +393,10 @@ __device__ __forceinline__ uint32_t job_bvh(const JobDev* jobs, uint32_t j, cons
 template <int LAYOUT>
 struct WaveSrc {
     using Index = uint32_t;
-    const float4* rays;  // this and the next two: written by the kernel before this one (launch.cuh)
+    const float4* rays;  // this and the next three: written by the kernel before this one (launch.cuh)
     const float4* srays;
-    const float4* con;
+    const float2* con;
+    const uint32_t* spid;
     float4* hits;
     float4* acc;
     const JobDev* jobs;
@@ -420,12 +421,14 @@ struct WaveSrc {
             return;
         }
         if (l.best_prim != 0xFFFFFFFFu) return;
-        const float4 c = con[i - nclosest];
-        const uint32_t pid = __float_as_uint(c.w);
+        const uint32_t k = i - nclosest;
+        const float r = srays[2ull * k + 1].z;
+        const float2 gb = con[k];
+        const uint32_t pid = spid[k];
         float4 a = acc[pid];
-        a.x += c.x;
-        a.y += c.y;
-        a.z += c.z;
+        a.x += r;
+        a.y += gb.x;
+        a.z += gb.y;
         acc[pid] = a;
     }
 };
@@ -436,7 +439,7 @@ __global__ void __launch_bounds__(trav::kMaxTraceThreads, 4) k_trace_wave(Paths 
     wait_for_previous();
     if (b > (int)ps.hdr->max_depth) return;
     const uint32_t nc = ps.cnt[b], ns = b ? ps.cnt[kShadowBase + b - 1] : 0u;
-    WaveSrc<LAYOUT> src{(b & 1) ? ps.ray[1] : ps.ray[0], ps.sray, ps.scon, ps.hit, ps.acc, ps.jobs, nc, nc + ns,
+    WaveSrc<LAYOUT> src{(b & 1) ? ps.ray[1] : ps.ray[0], ps.sray, ps.scon, ps.spid, ps.hit, ps.acc, ps.jobs, nc, nc + ns,
                         b == 0 ? kCameraTmin : kScatterTmin, b == 0 ? kCameraTmax : kScatterTmax};
     trav::traverse_loop<trav::kMixed, LAYOUT, SSTACK, trav::kRefillQueue>(
         src, trav::lanes_per_warp(src.n, gridDim.x * (blockDim.x / 32)), ps.work + b, &ps.hdr->err, s_stack);
@@ -550,7 +553,9 @@ __global__ void __launch_bounds__(kShadeThreads, 4) k_shade(Paths ps, int b, Pcg
     for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += stride) {
         const uint32_t i = base + threadIdx.x;
         bool scatter = false, shadow = false;
-        float4 new_r0, new_r1, sh_r0, sh_r1, sh_c;
+        float4 new_r0, new_r1, sh_r0, sh_r1;
+        float2 sh_c;
+        uint32_t sh_pid;
         float4 new_thr;
         if (i < n) {
             uint32_t e = i;  // queue entry
@@ -647,8 +652,9 @@ __global__ void __launch_bounds__(kShadeThreads, 4) k_shade(Paths ps, int b, Pcg
                                 const V3 so = sf.p - rd * 1.0e-4f;
                                 const V3 sd = lp - so;
                                 sh_r0 = make_float4(so.x, so.y, so.z, sd.x);
-                                sh_r1 = make_float4(sd.y, sd.z, 0.0f, r1.w);
-                                sh_c = make_float4(c.x, c.y, c.z, __uint_as_float(pid));
+                                sh_r1 = make_float4(sd.y, sd.z, c.x, r1.w);
+                                sh_c = make_float2(c.y, c.z);
+                                sh_pid = pid;
                                 shadow = true;
                             }
                         }
@@ -674,6 +680,7 @@ __global__ void __launch_bounds__(kShadeThreads, 4) k_shade(Paths ps, int b, Pcg
             ps.sray[2ull * sslot] = sh_r0;
             ps.sray[2ull * sslot + 1] = sh_r1;
             ps.scon[sslot] = sh_c;
+            ps.spid[sslot] = sh_pid;
         }
         if (scatter) {
             rays_next[2ull * nslot] = new_r0;
@@ -863,7 +870,8 @@ size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 // a wave's header fields and job table as the host stages them
 constexpr size_t kWaveBytes = (sizeof(WaveHeader) + sizeof(JobDev) * kMaxJobs + 255) & ~size_t(255);
 
-size_t path_layout(uint32_t cap, char* base, Paths* ps) {
+// grouped: with the arrays of the shading groups.
+size_t path_layout(uint32_t cap, bool grouped, char* base, Paths* ps) {
     size_t off = 0;
     auto take = [&](size_t bytes) {
         char* p = base ? base + off : nullptr;
@@ -875,9 +883,10 @@ size_t path_layout(uint32_t cap, char* base, Paths* ps) {
     for (int k = 0; k < 2; ++k) ps->thr[k] = (float4*)take(16 * c);
     ps->hit = (float4*)take(16 * c);
     ps->acc = (float4*)take(16 * c);
-    ps->bins = (uint32_t*)take(4 * ((kShadeBins + 1) / 2) * c);
     ps->sray = (float4*)take(32 * c);
-    ps->scon = (float4*)take(16 * c);
+    ps->scon = (float2*)take(8 * c);
+    ps->spid = (uint32_t*)take(4 * c);
+    ps->bins = grouped ? (uint32_t*)take(4 * ((kShadeBins + 1) / 2) * c) : nullptr;
     ps->cnt = (uint32_t*)take(kCounterBytes);  // counters and work counters, cleared as one
     ps->work = ps->cnt + kCntWords;
     ps->hdr = (WaveHeader*)take(sizeof(WaveHeader) + sizeof(JobDev) * kMaxJobs);
@@ -927,13 +936,18 @@ cudaError_t WavePool::ensure(uint32_t paths) {
     if (paths <= capacity && mem.p) return cudaSuccess;
     release_graphs();  // a captured wave points into the old path memory
     Paths p;
-    const size_t bytes = path_layout(paths, nullptr, &p);
-    e = mem.ensure(bytes);
+    bool grouped = true;
+    e = mem.ensure(path_layout(paths, true, nullptr, &p));
+    if (e == cudaErrorMemoryAllocation) {
+        (void)cudaGetLastError();
+        grouped = false;
+        e = mem.ensure(path_layout(paths, false, nullptr, &p));
+    }
     if (e != cudaSuccess) {
         capacity = 0;
         return e;
     }
-    path_layout(paths, (char*)mem.p, &ps);
+    path_layout(paths, grouped, (char*)mem.p, &ps);
     capacity = paths;
     return cudaMemset(ps.hdr, 0, sizeof(WaveHeader));
 }
@@ -1043,7 +1057,7 @@ cudaError_t run_wave(WavePool& pool, const JobDev* h_jobs, uint32_t njobs, uint3
     // shade in material groups when a large wave's scenes mix material types
     uint32_t types = 0;
     for (uint32_t j = 0; j < njobs; ++j) types |= h_jobs[j].sc.mat_types;
-    const bool bin = __builtin_popcount(types) >= 2 && total_paths > kQueueOrderPaths;
+    const bool bin = __builtin_popcount(types) >= 2 && total_paths > kQueueOrderPaths && ps.bins;
     const bool small = total_paths <= kOverlapPaths;
     if (!use_graph) return issue_wave(ps, max_depth, tgrid, sgrid, bin, small, s, tune);
     uint64_t key = 0x51ED270B27A3C1F5ull;

@@ -126,7 +126,8 @@ static_assert(sizeof(WaveHeader) == 48 && alignof(JobDev) <= 16, "the job table 
 // 256 x 256 x 16 spp 1,572 -> 1,524 us. Two buffers alternate by bounce. The RNG state is not stored: a path
 // that is alive has drawn the same count of numbers as every other path of its
 // bounce, so the state follows from (seed, pixel, sample) by one jump. Bytes
-// per path: 64 + 32 + 16 + 16 + 12 + 32 + 16 = 188.
+// per path: 64 + 32 + 16 + 16 + 32 + 12 = 172, and 12 for the shading groups
+// where there is room for them.
 struct Paths {
     // 2 per queue entry: (o.xyz, d.x), (d.y, d.z, path id bits, job bits); the
     // interval is a bounce's constant (camera rays 0 .. 1e34, scattered rays
@@ -138,10 +139,14 @@ struct Paths {
     float4* hit;    // per queue entry: (t, prim bits, u, v)
     float4* acc;    // per path id: (radiance rgb, 0)
     // the bounce's queue entries grouped for shading: group k in array k / 2,
-    // from its front when k is even, from its back when k is odd
+    // from its front when k is even, from its back when k is odd; null when
+    // memory lacked (waves then shade in queue order)
     uint32_t* bins;
-    float4* sray;   // shadow rays, 2 per entry: (o.xyz, d.x), (d.y, d.z, 0, job bits); interval 0 .. 0.9999
-    float4* scon;   // shadow contribution (rgb, path id bits)
+    // shadow rays, 2 per entry: (o.xyz, d.x), (d.y, d.z, contribution r, job bits);
+    // interval 0 .. 0.9999. The rest of the contribution and the path id are apart.
+    float4* sray;
+    float2* scon;   // shadow contribution (g, b)
+    uint32_t* spid; // path id
     uint32_t* cnt;  // [0, kMaxDepth]: closest queue sizes; [kMaxDepth+1, ...]: shadow queue sizes
     uint32_t* work;  // dynamic-fetch counters, one per trace launch of a wave
     WaveHeader* hdr;
@@ -189,7 +194,7 @@ struct WavePool {
 };
 
 // Paths per wave when the caller and the scene leave it open: a whole render
-// of up to 64 Mi paths (about 12.6 GB of path state) runs as one wave, which
+// of up to 64 Mi paths (about 12.3 GB of path state) runs as one wave, which
 // on the glossy 1024 x 768 x 64-spp render measured 80 ms against 108 ms in
 // 8 Mi-path waves (per-wave costs: the tails of 17 bounce steps, the resolve).
 constexpr uint32_t kDefaultWavePaths = 1u << 26;

@@ -61,7 +61,8 @@ typedef struct gr_bvh gr_bvh;
 typedef struct gr_opts {
     uint32_t default_wave_paths; /* paths in flight per render wave when neither the call nor its scene sets the
                                     wave size (0 = the whole call as one wave up to 64 Mi paths); the context's
-                                    pool of path state, about 188 bytes per path, grows to the largest wave used */
+                                    pool of path state, about 172 bytes per path and 12 more where there is room,
+                                    grows to the largest wave used */
     uint32_t flags;              /* reserved, 0 */
 } gr_opts;
 
@@ -413,8 +414,9 @@ int gr_scene_layout(const gr_scene* scene);
  * paths, and keeps the fastest as the scene's configuration and default wave
  * size. Images do not depend on any of these. Clears the scene's
  * accumulation. gr_render and gr_render_batch keep their path state in one
- * pool per context, sized by the largest wave asked of it (about 188 bytes
- * per path). */
+ * pool per context, sized by the largest wave asked of it (about 172 bytes
+ * per path, and 12 more where there is room, with which large waves of several
+ * material types are shaded in groups). */
 gr_status gr_scene_autotune(gr_scene* scene, const gr_render_opts* probe, gr_trace_tuning* best,
                             uint32_t* best_wave_paths);
 
