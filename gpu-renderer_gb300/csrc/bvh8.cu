@@ -589,17 +589,29 @@ cudaError_t bvh8_build(BvhBuffers& b, uint32_t n, DevBuf& scratch, int num_sms, 
     if (h.failed & ERR_TIMEOUT) return cudaErrorLaunchTimeout;
     if (h.overflow || h.failed) return cudaErrorInvalidValue;
     if (h.nodes > B.cap) {  // the layout's array grows: what it held stays in place
+        const auto copy = [&](Node8Q* to, const void* from, uint32_t count) {
+            return count ? cudaMemcpyAsync(to, from, sizeof(Node8Q) * count, cudaMemcpyDeviceToDevice, s) : cudaSuccess;
+        };
+        const size_t bytes = sizeof(Node8Q) * h.nodes;
         DevBuf grown;
-        if ((e = grown.ensure(sizeof(Node8Q) * h.nodes)) != cudaSuccess) return e;
-        if (B.cap && (e = cudaMemcpyAsync(grown.p, b.nodes8.p, sizeof(Node8Q) * B.cap, cudaMemcpyDeviceToDevice, s)) !=
-                         cudaSuccess)
+        e = grown.ensure(bytes);
+        if (e == cudaSuccess) {
+            if ((e = copy((Node8Q*)grown.p, b.nodes8.p, B.cap)) != cudaSuccess) return e;
+            if ((e = copy((Node8Q*)grown.p + B.cap, B.rest + B.cap, h.nodes - B.cap)) != cudaSuccess) return e;
+            if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return e;
+            std::swap(grown.p, b.nodes8.p);
+            std::swap(grown.bytes, b.nodes8.bytes);
+        } else if (e == cudaErrorMemoryAllocation && B.cap) {
+            // no room for both arrays: the old one's nodes wait in the scratch, whose first nodes are unused
+            (void)cudaGetLastError();
+            if ((e = copy(B.rest, b.nodes8.p, B.cap)) != cudaSuccess) return e;
+            if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return e;
+            if ((e = b.nodes8.ensure(bytes)) != cudaSuccess) return e;  // frees the old array first
+            if ((e = copy((Node8Q*)b.nodes8.p, B.rest, h.nodes)) != cudaSuccess) return e;
+            if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return e;
+        } else {
             return e;
-        if ((e = cudaMemcpyAsync((Node8Q*)grown.p + B.cap, B.rest + B.cap, sizeof(Node8Q) * (h.nodes - B.cap),
-                                 cudaMemcpyDeviceToDevice, s)) != cudaSuccess)
-            return e;
-        if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return e;
-        std::swap(grown.p, b.nodes8.p);
-        std::swap(grown.bytes, b.nodes8.bytes);
+        }
     }
     b.count8 = h.nodes;
     b.tris8_count = h.tris;

@@ -83,3 +83,40 @@ def test_nodes_that_found_no_memory_are_not_traversed(oracle):
     np.testing.assert_array_equal(d_hits.cpu().numpy().view(np.uint32), want)
     b.close()
     ctx.close()
+
+
+def test_nodes_grow_where_two_arrays_do_not_fit(oracle):
+    """A rebuild with more triangles on a GPU with room for the larger node array in the smaller one's place, not beside it
+    (everything else that the rebuild needs has grown before, but for the triangle array)."""
+    import torch
+    ctx = gr.Context(0)
+    n, m = 2000000, 1400000
+    v = sc.triangle_soup(n, seed_salt=886)
+    verts = torch.from_numpy(v).cuda()
+    rays = sc.incoherent_rays(1000, seed_salt=887)
+    d_rays, d_hits = torch.from_numpy(rays).cuda(), torch.zeros(1000, 4, dtype=torch.float32, device="cuda")
+    tree = oracle.lbvh(v)
+    nodes, tris = oracle.bvh8(tree)
+    other = gr.BVH(ctx)
+    other.set_layout(gr.LAYOUT_BVH8_Q8)
+    other.build_device(verts, n)  # the context's memory for 8-wide builds
+    other.close()
+    b = gr.BVH(ctx)
+    b.build_device(verts, n)
+    b.build_device(verts, m)
+    b.set_layout(gr.LAYOUT_BVH8_Q8)
+    small, small_tris = b.layout_size(gr.LAYOUT_BVH8_Q8)
+    grow_tris = tris.nbytes - small_tris
+    assert nodes.nbytes > small > (16 << 20)
+    held = fill_gpu(grow_tris + nodes.nbytes - small // 2)
+    try:
+        b.build_device(verts, n)
+        b.trace_device(d_rays, 1000, d_hits)
+        torch.cuda.synchronize()
+    finally:
+        del held
+        torch.cuda.empty_cache()
+    np.testing.assert_array_equal(b.export_layout(gr.LAYOUT_BVH8_Q8), nodes)
+    np.testing.assert_array_equal(d_hits.cpu().numpy().view(np.uint32), oracle.trace(tree, rays).view(np.uint32))
+    b.close()
+    ctx.close()
