@@ -155,6 +155,7 @@ struct BvhBuffers {
     uint32_t count8 = 0;             // 8-wide nodes
     uint32_t tris8_count = 0;        // triangles in tris8
     DevBuf scratch;                  // transient build state
+    bool scratch_clear = false;      // its block count (Scratch::done) has been set to zero
     DevBuf meta;                     // small device header (root, error word, centroid bounds)
 };
 

@@ -1240,7 +1240,14 @@ cudaError_t lbvh_build(BvhBuffers& b, const float* d_verts, uint32_t n, int num_
     const size_t had = b.scratch.p ? b.scratch.bytes : 0;
     if ((e = b.scratch.ensure(need)) != cudaSuccess) return e;
     scratch_layout(n, (char*)b.scratch.p, &s);
-    if (b.scratch.bytes != had && (e = cudaMemsetAsync(s.done, 0, 4, st)) != cudaSuccess) return e;  // new memory
+    if (b.scratch.bytes != had) b.scratch_clear = false;  // new memory
+    if (!b.scratch_clear) {
+        // a captured memset has not run yet, and may never: the next build sets it again
+        cudaStreamCaptureStatus capture;
+        if ((e = cudaStreamIsCapturing(st, &capture)) != cudaSuccess) return e;
+        if ((e = cudaMemsetAsync(s.done, 0, 4, st)) != cudaSuccess) return e;
+        b.scratch_clear = capture == cudaStreamCaptureStatusNone;
+    }
     return launch_build(d_verts, n, s, (Node*)b.nodes.p, (Tri*)b.tris.p, (uint32_t*)b.code.p, (uint32_t*)b.prim.p,
                         meta, num_sms, st);
 }

@@ -118,3 +118,39 @@ def test_small_waves_back_to_back(ctx, layout):
             np.testing.assert_array_equal(a, b)
     for s in scenes:
         s.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("replay", [False, True])
+def test_a_captured_first_build_leaves_the_next_one_sound(ctx, oracle, replay):
+    """The first build of a BVH, which allocates, recorded into a graph; the next one runs at once, whether the graph has been
+    launched or not. The memory that the BVH gets held other values before."""
+    import torch
+    n = 3001
+    v, w = sc.triangle_soup(n, seed_salt=920), sc.triangle_soup(n, seed_salt=921)
+    dv, dw = (torch.from_numpy(x.reshape(n, 9)).cuda() for x in (v, w))
+    for size in (1 << 12, 1 << 16, 1 << 18, 1 << 20, 1 << 26):
+        dirty = [torch.full((size,), 255, dtype=torch.uint8, device="cuda") for _ in range(4)]
+        torch.cuda.synchronize()
+        del dirty
+    torch.cuda.empty_cache()
+    b, st, g = gr.BVH(ctx), torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    warm = gr.BVH(ctx)
+    warm.build_device(dv, n)  # kernels loaded
+    torch.cuda.synchronize()
+    with torch.cuda.graph(g, stream=st, capture_error_mode="relaxed"):
+        b.build_device(dv, n, stream=torch.cuda.current_stream().cuda_stream)
+    steps = [lambda: b.build_device(dw, n, stream=st.cuda_stream)]
+    want = [oracle.lbvh(w)]
+    if replay:
+        steps = [g.replay] + steps + [g.replay]
+        want = [oracle.lbvh(v)] + want + [oracle.lbvh(v)]
+    for step, tree in zip(steps, want):
+        with torch.cuda.stream(st):
+            step()
+        st.synchronize()
+        got = b.export()
+        for k in ("root", "sorted_prim", "sorted_code", "nodes"):
+            np.testing.assert_array_equal(got[k], tree[k], err_msg=k)
+    warm.close()
+    b.close()
