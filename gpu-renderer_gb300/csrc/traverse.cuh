@@ -36,8 +36,12 @@ struct RayW {
 };
 
 __device__ __forceinline__ float pick(float x, float y, float z, int k) { return k == 0 ? x : (k == 1 ? y : z); }
-// The coordinate that bits `at`, `at` + 1 of RayW::axes name.
+// The coordinate that bits `at`, `at` + 1 of RayW::axes name; FIELDS: read as one number,
+// else bit by bit (the compiler's code differs: see tri_test).
+template <bool FIELDS>
 __device__ __forceinline__ float pick_axis(float x, float y, float z, uint32_t axes, int at) {
+    const uint32_t k = (axes >> at) & 3u;
+    if (FIELDS) return k == 1u ? x : (k == 2u ? y : z);
     return (axes & (1u << at)) ? x : ((axes & (2u << at)) ? y : z);
 }
 
@@ -117,7 +121,11 @@ __device__ __forceinline__ float2 sub2(float a0, float a1, float b0, float b1) {
 // roundings). Faster in the 8-wide kernels, whose leaf loop is a third of their
 // instructions (batch of 8 scenes 8.31 -> 8.21 ms, Cornell box 1,105 -> 1,098 us), slower
 // in the binary one, which waits for its nodes (786 k camera rays 1,026 -> 1,031 us).
-template <bool PACKED>
+// FIELDS: for the 4-wide any-hit kernels, which the bits made slower than three axis
+// numbers (700 k shadow rays in 270,001 triangles, quantised nodes: numbers 1,741 us, bits
+// 1,770, fields 1,739); their closest-hit kernels are the faster with bits (camera rays
+// 1,254, 1,226, 1,260).
+template <bool PACKED, bool FIELDS>
 __device__ __forceinline__ bool tri_test(const RayW& p, const float4 a, const float4 b, const float4 c, float tbest,
                                          float& t, float& u, float& v) {
     const auto xy = [&](const float4 q) {
@@ -127,13 +135,13 @@ __device__ __forceinline__ bool tri_test(const RayW& p, const float4 a, const fl
     const float Ax0 = A0.x, Ay0 = A0.y, Az0 = __fsub_rn(a.z, p.oz);
     const float Bx0 = B0.x, By0 = B0.y, Bz0 = __fsub_rn(b.z, p.oz);
     const float Cx0 = C0.x, Cy0 = C0.y, Cz0 = __fsub_rn(c.z, p.oz);
-    const float Akz = pick_axis(Ax0, Ay0, Az0, p.axes, 4), Bkz = pick_axis(Bx0, By0, Bz0, p.axes, 4), Ckz = pick_axis(Cx0, Cy0, Cz0, p.axes, 4);
-    const float Ax = __fmaf_rn(-p.sx, Akz, pick_axis(Ax0, Ay0, Az0, p.axes, 0));
-    const float Ay = __fmaf_rn(-p.sy, Akz, pick_axis(Ax0, Ay0, Az0, p.axes, 2));
-    const float Bx = __fmaf_rn(-p.sx, Bkz, pick_axis(Bx0, By0, Bz0, p.axes, 0));
-    const float By = __fmaf_rn(-p.sy, Bkz, pick_axis(Bx0, By0, Bz0, p.axes, 2));
-    const float Cx = __fmaf_rn(-p.sx, Ckz, pick_axis(Cx0, Cy0, Cz0, p.axes, 0));
-    const float Cy = __fmaf_rn(-p.sy, Ckz, pick_axis(Cx0, Cy0, Cz0, p.axes, 2));
+    const float Akz = pick_axis<FIELDS>(Ax0, Ay0, Az0, p.axes, 4), Bkz = pick_axis<FIELDS>(Bx0, By0, Bz0, p.axes, 4), Ckz = pick_axis<FIELDS>(Cx0, Cy0, Cz0, p.axes, 4);
+    const float Ax = __fmaf_rn(-p.sx, Akz, pick_axis<FIELDS>(Ax0, Ay0, Az0, p.axes, 0));
+    const float Ay = __fmaf_rn(-p.sy, Akz, pick_axis<FIELDS>(Ax0, Ay0, Az0, p.axes, 2));
+    const float Bx = __fmaf_rn(-p.sx, Bkz, pick_axis<FIELDS>(Bx0, By0, Bz0, p.axes, 0));
+    const float By = __fmaf_rn(-p.sy, Bkz, pick_axis<FIELDS>(Bx0, By0, Bz0, p.axes, 2));
+    const float Cx = __fmaf_rn(-p.sx, Ckz, pick_axis<FIELDS>(Cx0, Cy0, Cz0, p.axes, 0));
+    const float Cy = __fmaf_rn(-p.sy, Ckz, pick_axis<FIELDS>(Cx0, Cy0, Cz0, p.axes, 2));
     const float U = __fsub_rn(__fmul_rn(Cx, By), __fmul_rn(Cy, Bx));
     const float V = __fsub_rn(__fmul_rn(Ax, Cy), __fmul_rn(Ay, Cx));
     const float W = __fsub_rn(__fmul_rn(Bx, Ay), __fmul_rn(By, Ax));
@@ -197,12 +205,12 @@ __device__ __forceinline__ bool wants_any(const L_& L) {
 
 // Tests leaf triangle `c` (~sorted position); returns true when an any-hit
 // query is answered. Closest-hit ties at equal t go to the smaller prim id.
-template <int Q, bool PACKED = false, class L_>
+template <int Q, bool PACKED = false, bool FIELDS = false, class L_>
 __device__ __forceinline__ bool leaf(L_& L, int32_t c) {
     const Tri* tr = L.tris + (uint32_t)(~c);
     const float4 a = __ldg(&tr->a), b = __ldg(&tr->b), cc = __ldg(&tr->c);
     float t, u, v;
-    if (!tri_test<PACKED>(L.p, a, b, cc, L.best_t, t, u, v)) return false;
+    if (!tri_test<PACKED, FIELDS>(L.p, a, b, cc, L.best_t, t, u, v)) return false;
     const uint32_t prim = __float_as_uint(a.w);
     const bool any = wants_any<Q>(L);
     if (any || t < L.best_t || prim < L.best_prim) {
@@ -364,7 +372,7 @@ __device__ __forceinline__ bool trace_step4(L_& L, int2* s_stack, int2* l_stack,
             }
         if (!hr) continue;
         if (cr < 0) {
-            if (leaf<Q>(L, cr)) return true;
+            if (leaf<Q, false, Q == kAny>(L, cr)) return true;
         } else if (!have) {
             next = cr;
             have = true;
