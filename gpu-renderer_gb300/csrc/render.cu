@@ -442,7 +442,7 @@ __global__ void __launch_bounds__(trav::kMaxTraceThreads, 4) k_trace_wave(Paths 
     WaveSrc<LAYOUT> src{(b & 1) ? ps.ray[1] : ps.ray[0], ps.sray, ps.scon, ps.spid, ps.hit, ps.acc, ps.jobs, nc, nc + ns,
                         b == 0 ? kCameraTmin : kScatterTmin, b == 0 ? kCameraTmax : kScatterTmax};
     trav::traverse_loop<trav::kMixed, LAYOUT, SSTACK, trav::kRefillQueue>(
-        src, trav::lanes_per_warp(src.n, gridDim.x * (blockDim.x / 32)), ps.work + b, &ps.hdr->err, s_stack);
+        src, trav::lanes_per_warp(LAYOUT, src.n, gridDim.x * (blockDim.x / 32)), ps.work + b, &ps.hdr->err, s_stack);
 }
 
 // ---- shading groups -----------------------------------------------------------------

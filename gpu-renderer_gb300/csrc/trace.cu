@@ -81,7 +81,7 @@ cudaError_t launch(const BvhDevice& bvh, const void* nodes, int block, const flo
         if (occ[bi] < 1) occ[bi] = 1;
     }
     const uint32_t warps = (uint32_t)(num_sms * occ[bi] * (block / 32));
-    const uint32_t lanes = trav::lanes_per_warp(n, warps);
+    const uint32_t lanes = trav::lanes_per_warp(LAYOUT, n, warps);
     const uint64_t warps_needed = (n + lanes - 1) / lanes;
     const uint64_t blocks_needed = (warps_needed + block / 32 - 1) / (block / 32);
     const uint64_t resident = (uint64_t)num_sms * occ[bi] * trav::resident_eighths(LAYOUT, n, warps) / 8;
