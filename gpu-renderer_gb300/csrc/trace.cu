@@ -81,7 +81,11 @@ cudaError_t launch(const BvhDevice& bvh, const void* nodes, int block, const flo
         if (occ[bi] < 1) occ[bi] = 1;
     }
     const uint32_t warps = (uint32_t)(num_sms * occ[bi] * (block / 32));
-    const uint32_t lanes = trav::lanes_per_warp(LAYOUT, n, warps);
+    // A tree of one or two levels is not worth more warps: 10,000 rays, one triangle, binary
+    // nodes 6.9 us with 32 lanes and 8.4 spread, 8-wide nodes 8.3 and 9.5; from 8 triangles
+    // (16 in 8-wide nodes) on, spreading is faster (16, 1,000 rays, binary: 14.2 and 10.5).
+    const bool flat = bvh.n <= (LAYOUT == kLayoutBvh8Q8 ? 8u : 4u);
+    const uint32_t lanes = flat ? 32u : trav::lanes_per_warp(LAYOUT, n, warps);
     const uint64_t warps_needed = (n + lanes - 1) / lanes;
     const uint64_t blocks_needed = (warps_needed + block / 32 - 1) / (block / 32);
     const uint64_t resident = (uint64_t)num_sms * occ[bi] * trav::resident_eighths(LAYOUT, n, warps) / 8;
