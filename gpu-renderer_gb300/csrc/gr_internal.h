@@ -186,7 +186,7 @@ cudaError_t lbvh_build_static(const float* d_verts, uint32_t n, Node* nodes, Tri
 cudaError_t bvh4_build(BvhBuffers& b, uint32_t n, int layout, cudaStream_t s);
 // bvh8.cu: all levels in one cooperative launch; waits for `s` to read the sizes.
 // cudaErrorLaunchTimeout when a barrier gave up, here or in the binary build.
-// `scratch` holds the build's state (about 144 bytes per triangle); it is the
+// `scratch` holds the build's state (136 bytes per triangle); it is the
 // context's, kept between builds, and the caller holds its lock.
 cudaError_t bvh8_build(BvhBuffers& b, uint32_t n, DevBuf& scratch, int num_sms, cudaStream_t s);
 

@@ -841,7 +841,8 @@ __device__ __forceinline__ bool load_sub(const Sub* ps, Sub& s) {
 // finished, about 1 us a level instead of 2. Build times, climbing over the whole
 // GPU against in one block: 300 triangles 54 / 48 us, 3,001 70 / 56, 10,000 85 / 70,
 // 100,003 99 / 93, 131,072 105 / 101; at 1 M the one block's throughput is the limit
-// (192 / 365 us with the siblings met through L2).
+// (192 / 365 us with the siblings met through L2). Between the two it is not measured: the
+// line is where the block's 48 KB of shared memory end.
 constexpr uint32_t kBlockClimbChunks = 512;
 constexpr int kBlockClimbThreads = 1024;
 constexpr uint32_t kSpreadChunks = 64;
@@ -1113,8 +1114,8 @@ cudaError_t sort_coop_capacity(int num_sms, int* tiles) {
 // Keys a thread of the cooperative sort ranks (tiles of 512 times that). A pass
 // lasts as long as its busiest SM, and ranking is most of it, so tiles are as small
 // as a limit on their number allows: one tile, which has no barriers, up to 3,072
-// keys (3,001 triangles built in 37.8 us, in several tiles 39.8; 4,000 in 41.9 and
-// 39.9); else kSumTiles, beyond which the counts take a scan and a barrier more a
+// keys (one tile against several: 1,600 triangles 31.0 / 36.9 us, 2,500 33.9 / 35.3,
+// 3,072 36.7 / 37.3, 3,500 39.1 / 40.2, 4,000 41.0 / 38.6); else kSumTiles, beyond which the counts take a scan and a barrier more a
 // pass (98,304 triangles: 64 tiles 70.7, 96 tiles 77.9); else one tile an SM; else
 // what is resident. Builds with this rule against 8 keys a thread always (us):
 // 600 triangles 37 / 29, 5,000 47 / 39, 30,000 61 / 49, 100,003 80 / 71, 131,072

@@ -1052,7 +1052,7 @@ cudaError_t run_wave(WavePool& pool, const JobDev* h_jobs, uint32_t njobs, uint3
     const int tgrid = num_sms * occ;
     const int sgrid = num_sms * 4;
     // the captured sequence runs exactly the wave's bounce steps (an empty step
-    // still costs three launches)
+    // still costs its two or three launches)
     const uint32_t steps = max_depth;
     // shade in material groups when a large wave's scenes mix material types
     uint32_t types = 0;

@@ -37,8 +37,8 @@ struct DevCamera {
 // Camera::setup (camera.h:21-38) from the C-ABI record.
 DevCamera make_camera(const gr_camera& c);
 
-// One emissive triangle as light sampling reads it: five 16-byte loads at an
-// address known from the light's index (through the light list, the triangle's
+// One emissive triangle as light sampling reads it: four 16-byte loads and one word
+// at an address known from the light's index (through the light list, the triangle's
 // vertices and its material they were three dependent steps, and its area and
 // normal were computed for every sample; with the other cuts of its commit,
 // k_shade's bounce 0 of the glossy 1024 x 768 x 64 spp render 4.42 -> 3.38 ms).
@@ -195,8 +195,9 @@ struct WavePool {
 
 // Paths per wave when the caller and the scene leave it open: a whole render
 // of up to 64 Mi paths (about 12.3 GB of path state) runs as one wave, which
-// on the glossy 1024 x 768 x 64-spp render measured 80 ms against 108 ms in
-// 8 Mi-path waves (per-wave costs: the tails of 17 bounce steps, the resolve).
+// on the glossy 1024 x 768 x 64-spp render measures 53 ms against 67 ms in
+// 8 Mi-path waves and 56 ms in 32 Mi ones (per-wave costs: the tails of 17
+// bounce steps, the resolve).
 constexpr uint32_t kDefaultWavePaths = 1u << 26;
 
 // The path pool of a context's gr_render and gr_render_batch calls (created on
@@ -241,11 +242,11 @@ namespace gr {
 uint32_t pack_wave(std::vector<HostJob*>& jobs, uint32_t capacity, std::vector<JobDev>& out, uint32_t* total_paths,
                    uint32_t* total_pix, uint32_t* max_depth);
 
-// Mean radiance -> sRGB-encoded RGBA8 (R in the low byte), the reference's
-// filter_kernel (pathtracer_kernel.h:792-810); pixels without samples are black.
 // The light records of a scene view (its lights, triangles and materials set) into `out`.
 cudaError_t light_records(const SceneDev& sc, LightDev* out, cudaStream_t s);
 
+// Mean radiance -> sRGB-encoded RGBA8 (R in the low byte), the reference's
+// filter_kernel (pathtracer_kernel.h:792-810); pixels without samples are black.
 cudaError_t filter_rgba8(const double* fb, const uint32_t* fbc, uint32_t npix, uint32_t* out, cudaStream_t s);
 // Mean radiance of an accumulation into 3 floats per pixel in memory the device
 // can write (device memory, or page-locked host memory).

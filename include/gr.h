@@ -68,7 +68,7 @@ typedef struct gr_opts {
 
 /* Binds `device` and creates a context (streams, memory pool); `opts` may be
  * NULL for the defaults. The context keeps the 8-wide layout build's scratch
- * (about 144 bytes per triangle of the largest BVH it has collapsed) between
+ * (136 bytes per triangle of the largest BVH it has collapsed) between
  * builds, so building a layout neither allocates nor frees device memory once
  * it has grown; destroying the context frees it. Replaces the process-global
  * CUDA state the reference sets up implicitly. */
