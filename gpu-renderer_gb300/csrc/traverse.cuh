@@ -656,7 +656,7 @@ __host__ __device__ constexpr int steps_per_check(int layout) { return layout ==
 // against one ray for every resident warp first (us): binary nodes 1,021 rays
 // 192 / 119 / 119, 10,000 230 / 167 / 175, 50,000 242 / 226 / 247; 8-wide nodes
 // 1,021 rays 103 / 66 / 67, 10,000 126 / 105 / 112, 50,000 135 / 140 / 174. A
-// 160 x 120 x 1 spp preview 615 -> 460 us. 4-wide nodes, whose leaf tests are fewer, gain
+// 160 x 120 x 1 spp preview 615 -> 460 us. 4-wide nodes gain
 // only up to 8 lanes: shadow rays in 270,001 triangles, quantised, 32 lanes against the
 // others' rule (us): 10,000 rays 359 / 333, 20,000 381 / 389, 39,000 419 / 453, 50,000
 // 457 / 481.
